@@ -22,8 +22,8 @@
 #if MBM_FAST_ARITH
 #define MBM_HD __host__ __device__ __forceinline__
 #include "mbm_adjoint_math.cuh"   // primitive-form Conservative and Grad-13 flux
-#include "mbm_newton.cuh"
 #endif
+#include "mbm_newton.cuh"
 
 namespace mbm {
 namespace MBM_ARITH {
@@ -39,37 +39,31 @@ __device__ __forceinline__ double rsgn(double a) { return a == 0 ? 0.0 : (a < 0 
 // Markstein's correction step (P. Markstein, "Computation of elementary functions
 // on the IBM RISC System/6000 processor", IBM J. Res. Develop. 34(1):111-119, 1990;
 // J.-M. Muller et al., Handbook of Floating-Point Arithmetic, 2nd ed., 2018, ch. 4):
-// with r = RN(1/y) and q = RN(x*r), the remainder e = x - q*y is exact in one FMA
-// and RN(q + e*r) = RN(x/y), provided x, y and the quotient stay in the normal
+// with r = RN(1/y) and q = RN(x*r), the remainder q*y - x is exact in one FMA and
+// RN(q - (q*y - x)*r) = RN(x/y), provided x, y and the quotient stay in the normal
 // range.  One reciprocal then serves every quotient with the same denominator at
-// three FP64 operations each, with the same bits as IEEE x/y.  The quotient is
-// formed without a branch; a range flag (integer pipe only: |exponent| < 480 for
-// x and y, or x = 0) is collected per function, and a function whose flag is set
-// recomputes its quotients with IEEE division in a cold, outlined path.  Zero
-// numerators take x*r, the signed zero of x/y.  Checked against x/y on the host
-// for 2e8 random operand pairs and by every bitwise parity test.
+// three FP64 operations each, with the same bits as IEEE x/y.  For y > 0 the negated
+// remainder gives zeros their sign too: x = +-0 leaves q = +-0, the remainder q*y - x is
+// +0, and -(+0)*r + q = q.  The reciprocal is Markstein's as well: the hardware
+// approximation refined to within one unit in the last place (the third-order step of
+// mbm_newton.cuh), then RN(r + r(1 - y r)), which is RN(1/y) unless y's significand is
+// all ones (set apart).
+//
+// The hot path has no branch per quotient.  A set of quotients is checked together by
+// integer minima and maxima of its numerators' high words (MkRange: about four integer
+// instructions each, zeros admitted); a set with a numerator out of range, or whose
+// denominator is not positive or out of range, is divided by IEEE division, out of line.
+// Measured (bitwise step): 4 x 1024^2 cells, harmonic, 3.15 ms with a full test and a
+// signed-zero select per quotient (ten integer instructions) and IEEE divisions in the
+// limiter, 1.81 ms like this; 28 blocks of 30 x 10 in a stream, most sets holding a zero,
+// 143 against 129 us (checking exponents alone and sorting the zeros out in a second look:
+// 1.96 ms and 143 us).
+// Checked against x/y on the host for random and near-tie operands
+// (tests/test_division.py, tests/test_exact_division.py) and by every bitwise parity test.
 //
 // Fast arithmetic (MBM_FAST_ARITH, MBM_MODE_FAST): the quotient is RN(x*r) without
-// the correction, within one unit in the last place of x/y, and no range flag is
-// kept (the cold IEEE paths become dead code); the file is then compiled with
-// multiply-add contraction.
-#if MBM_FAST_ARITH
-__device__ __forceinline__ bool mk_in(double) { return true; }
-
-__device__ __forceinline__ double mk_div(double x, double, double r) { return x * r; }
-#else
-__device__ __forceinline__ bool mk_in(double x) {
-  const long long b = __double_as_longlong(x);
-  return (((unsigned)(b >> 52) & 0x7ffu) - 543u <= 960u) || ((b << 1) == 0);
-}
-
-__device__ __forceinline__ double mk_div(double x, double y, double r) {
-  const double q = x * r;
-  const double m = fma(fma(-q, y, x), r, q);
-  return ((__double_as_longlong(x) << 1) == 0) ? q : m;
-}
-#endif
-
+// the correction, within one unit in the last place of x/y, and nothing is checked; the
+// file is then compiled with multiply-add contraction.
 __device__ __noinline__ double div_ieee(double x, double y) { return x / y; }
 
 // Reciprocal, square root and lone quotients.  Bitwise: IEEE division and sqrt.
@@ -81,82 +75,107 @@ __device__ __forceinline__ double fdiv(double x, double y) { return x * frcp(y);
 #else
 __device__ __forceinline__ double fdiv(double x, double y) { return x / y; }
 __device__ __forceinline__ double fsqrt(double x) { return sqrt(x); }
+
+constexpr unsigned MK_LO = 543u << 21;             // 2^-480, as (high word << 1)
+constexpr unsigned MK_SPAN = (961u << 21) - 1u;    // up to 2^481, exclusive
+
+// The numerators of a set: in range if each is zero or has its exponent in the admitted
+// range.  (high word << 1) - 1 + (low word != 0) is all ones for a zero and keeps the
+// order of everything else, deep subnormals included, so its minimum finds the small ones.
+struct MkRange {
+  unsigned lo = ~0u, hi = 0u;
+  __device__ __forceinline__ void add(double x) {
+    const unsigned h = 2u * (unsigned)__double2hiint(x);
+    unsigned u;
+    asm("{\n .reg .u32 t;\n add.cc.u32 t, %1, 0xffffffff;\n addc.u32 %0, %2, 0xffffffff;\n}"
+        : "=r"(u) : "r"(__double2loint(x)), "r"(h));
+    lo = min(lo, u);
+    hi = max(hi, h);
+  }
+  __device__ __forceinline__ bool bad() const { return lo < MK_LO || hi > MK_LO + MK_SPAN; }
+};
+
+__device__ __forceinline__ double mk_div(double x, double y, double r) {   // y > 0
+  const double q = x * r;
+  return fma(-fma(q, y, -x), r, q);
+}
+
+// RN(1/y) for y in range, unless y's significand is all ones
+__device__ __forceinline__ double mk_rcp(double y) {
+  const double r = mbm_newton::frcp(y);
+  return fma(fma(-y, r, 1.0), r, r);
+}
+// a significand of all ones, y = 2^k (2 - 2^-52): then RN(1/y) = 2^(-k-1) (1 + 2^-52).
+// Densities one rounding below 1 make this an everyday value of a stream at rho = 1.
+__device__ __forceinline__ double mk_rcp_all(double y) {
+  const int h = __double2hiint(y);
+  const double r = mk_rcp(y);
+  return ((h | (int)0xfff00000) & __double2loint(y)) == -1
+             ? __hiloint2double((2045 << 20) - (h & 0x7ff00000), 1) : r;
+}
+// y not positive or out of range
+__device__ __forceinline__ bool mk_bad_den(double y) {
+  return (unsigned)__double2hiint(y) - (543u << 20) >= (961u << 20);
+}
 #endif
 
 struct Recip {        // 1/y for a denominator shared by several quotients
   double y, r;
-  bool bad;           // set when any quotient left the safe range
-  __device__ __forceinline__ explicit Recip(double y_) {
-    y = y_;
 #if MBM_FAST_ARITH
-    r = frcp(y_);
+  __device__ __forceinline__ explicit Recip(double y_) : y(y_), r(frcp(y_)) {}
+  __device__ __forceinline__ Recip(double y_, double r_) : y(y_), r(r_) {}
 #else
-    r = __drcp_rn(y_);
+  bool bad;           // y outside what mk_rcp and mk_div admit
+  __device__ __forceinline__ explicit Recip(double y_) : y(y_), r(mk_rcp_all(y_)), bad(mk_bad_den(y_)) {}
+  __device__ __forceinline__ Recip(double y_, double r_) : y(y_), r(r_), bad(false) {}   // r_ = RN(1/y_), y_ in range
 #endif
-#if MBM_FAST_ARITH
-    bad = false;      // no range check: quotients are x * r, no IEEE fallback
-#else
-    const unsigned e = (unsigned)(__double_as_longlong(y_) >> 52) & 0x7ffu;
-    bad = e - 543u > 960u;
-#endif
-  }
-  __device__ __forceinline__ Recip(double y_, double r_) {   // r_ = RN(1/y_), y_ in range
-    y = y_;
-    r = r_;
-    bad = false;
-  }
-  __device__ __forceinline__ double div(double x) {
-    bad |= !mk_in(x);
-    return mk_div(x, y, r);
-  }
-  __device__ __forceinline__ double exact(double x) const { return mk_div(x, y, r); }
 };
 
-struct V9 { double v[NV]; };
-
-// Primitive (src/Flux.c:30-56)
-__device__ __noinline__ V9 primitive_ieee(V9 u) {
-  const double* U = u.v;
-  V9 o;
-  double* P = o.v;
-  const double rho = U[0];
-  const double v1 = U[1] / rho, v2 = U[2] / rho;
-  const double vs = v1 * v1 + v2 * v2;
-  const double th = (2 * U[3] / rho - vs) / 3;
-  const double E = U[3];
-  const double T11 = U[4] / rho - v1 * v1;
-  const double T12 = U[5] / rho - v1 * v2;
-  const double T22 = U[6] / rho - v2 * v2;
-  P[0] = rho; P[1] = v1; P[2] = v2; P[3] = th;
-  P[4] = T11; P[5] = T12; P[6] = T22;
-  P[7] = U[7] - E * v1 - rho * (T11 * v1 + T12 * v2);
-  P[8] = U[8] - E * v2 - rho * (T12 * v1 + T22 * v2);
-  return o;
+// q[n] = x[n] / D.y
+template <int N>
+__device__ __forceinline__ void quotients(const double (&x)[N], const Recip& D, double (&q)[N]) {
+#if MBM_FAST_ARITH
+#pragma unroll
+  for (int n = 0; n < N; n++) q[n] = x[n] * D.r;
+#else
+  MkRange g;
+#pragma unroll
+  for (int n = 0; n < N; n++) {
+    g.add(x[n]);
+    q[n] = mk_div(x[n], D.y, D.r);
+  }
+  if (__builtin_expect(g.bad() || D.bad, 0)) {
+#pragma unroll
+    for (int n = 0; n < N; n++) q[n] = div_ieee(x[n], D.y);
+  }
+#endif
 }
 
+__device__ __forceinline__ double quotient(double x, const Recip& D) {
+  const double a[1] = {x};
+  double q[1];
+  quotients(a, D, q);
+  return q[0];
+}
+
+// Primitive (src/Flux.c:30-56)
 __device__ __forceinline__ void primitive(const double (&U)[NV], double (&P)[NV]) {
   const double rho = U[0];
-  Recip R(rho);
-  Recip third(3.0, 1.0 / 3.0);
-  const double v1 = R.div(U[1]), v2 = R.div(U[2]);
+  const Recip R(rho), third(3.0, 1.0 / 3.0);
+  const double x[6] = {U[1], U[2], 2 * U[3], U[4], U[5], U[6]};
+  double q[6];
+  quotients(x, R, q);
+  const double v1 = q[0], v2 = q[1];
   const double vs = v1 * v1 + v2 * v2;
-  const double th = third.div(R.div(2 * U[3]) - vs);
+  const double th = quotient(q[2] - vs, third);
   const double E = U[3];
-  const double T11 = R.div(U[4]) - v1 * v1;
-  const double T12 = R.div(U[5]) - v1 * v2;
-  const double T22 = R.div(U[6]) - v2 * v2;
+  const double T11 = q[3] - v1 * v1;
+  const double T12 = q[4] - v1 * v2;
+  const double T22 = q[5] - v2 * v2;
   P[0] = rho; P[1] = v1; P[2] = v2; P[3] = th;
   P[4] = T11; P[5] = T12; P[6] = T22;
   P[7] = U[7] - E * v1 - rho * (T11 * v1 + T12 * v2);
   P[8] = U[8] - E * v2 - rho * (T12 * v1 + T22 * v2);
-  if (__builtin_expect(R.bad || third.bad, 0)) {
-    V9 u;
-#pragma unroll
-    for (int n = 0; n < NV; n++) u.v[n] = U[n];
-    const V9 o = primitive_ieee(u);
-#pragma unroll
-    for (int n = 0; n < NV; n++) P[n] = o.v[n];
-  }
 }
 
 // moments with an explicit energy (src/Flux.c:65-73, 255-263)
@@ -181,27 +200,27 @@ __device__ __forceinline__ void conservative(const double (&P)[NV], double (&U)[
   moments_e(P[0], P[1], P[2], E, P[4], P[5], P[6], P[7], P[8], U);
 }
 
-// Grad-13 flux along x of a moment vector (src/Flux.c:79-119).  D: the division
-// policy -- shared reciprocals (fast) or IEEE (cold path).
-template <bool IEEE>
-__device__ __forceinline__ bool grad13_flux_x_t(const double (&U)[NV], double (&F)[NV]) {
+#if !MBM_FAST_ARITH
+// Grad-13 flux along x of a moment vector (src/Flux.c:79-119)
+__device__ __forceinline__ void grad13_flux_x(const double (&U)[NV], double (&F)[NV]) {
   const double rho = U[0];
-  Recip R(rho);
-  Recip third(3.0, 1.0 / 3.0);
-#define MBM_DIV(D, x) (IEEE ? (x) / D.y : D.div(x))
-  const double v1 = MBM_DIV(R, U[1]), v2 = MBM_DIV(R, U[2]);
+  const Recip R(rho), third(3.0, 1.0 / 3.0);
+  const double x[6] = {U[1], U[2], 2 * U[3], U[4], U[5], U[6]};
+  double q[6];
+  quotients(x, R, q);
+  const double v1 = q[0], v2 = q[1];
   const double vs = v1 * v1 + v2 * v2;
-  const double th = MBM_DIV(third, MBM_DIV(R, 2 * U[3]) - vs);
+  const double th = quotient(q[2] - vs, third);
   const double E = U[3];
-  const double T11 = MBM_DIV(R, U[4]) - v1 * v1;
-  const double T12 = MBM_DIV(R, U[5]) - v1 * v2;
-  const double T22 = MBM_DIV(R, U[6]) - v2 * v2;
+  const double T11 = q[3] - v1 * v1;
+  const double T12 = q[4] - v1 * v2;
+  const double T22 = q[5] - v2 * v2;
   const double q1 = U[7] - E * v1 - rho * (T11 * v1 + T12 * v2);
   const double q2 = U[8] - E * v2 - rho * (T12 * v1 + T22 * v2);
-  const double M111 = MBM_DIV(R, 1.2 * q1);
-  const double M121 = MBM_DIV(R, 0.4 * q2), M112 = M121;
-  const double M221 = MBM_DIV(R, 0.4 * q1), M122 = M221;
-#undef MBM_DIV
+  const double y[3] = {1.2 * q1, 0.4 * q2, 0.4 * q1};
+  double M[3];
+  quotients(y, R, M);
+  const double M111 = M[0], M121 = M[1], M112 = M[1], M221 = M[2], M122 = M[2];
   const double R11 = 5 * th * th + 7 * th * (T11 - th);
   const double R12 = 7 * th * T12;
   F[0] = rho * v1;
@@ -215,85 +234,98 @@ __device__ __forceinline__ bool grad13_flux_x_t(const double (&U)[NV], double (&
          rho * (M111 * v1 + M112 * v2) + 0.5 * rho * (T11 * vs + R11);
   F[8] = q2 * v1 + q1 * v2 + rho * (v1 * v2 * (T11 + T22) + 1.5 * T12 * vs) + E * v1 * v2 +
          rho * (M121 * v1 + M122 * v2) + 0.5 * rho * R12;
-  return IEEE ? false : (R.bad || third.bad);
 }
 
-__device__ __noinline__ V9 grad13_flux_x_ieee(V9 u) {
-  double U[NV], F[NV];
-#pragma unroll
-  for (int n = 0; n < NV; n++) U[n] = u.v[n];
-  grad13_flux_x_t<true>(U, F);
-  V9 o;
-#pragma unroll
-  for (int n = 0; n < NV; n++) o.v[n] = F[n];
-  return o;
-}
-
-__device__ __forceinline__ void grad13_flux_x(const double (&U)[NV], double (&F)[NV]) {
-  if (__builtin_expect(grad13_flux_x_t<false>(U, F), 0)) {
-    V9 u;
-#pragma unroll
-    for (int n = 0; n < NV; n++) u.v[n] = U[n];
-    const V9 o = grad13_flux_x_ieee(u);
-#pragma unroll
-    for (int n = 0; n < NV; n++) F[n] = o.v[n];
-  }
+// a*c + b*d with one of c, d +-1 and the other +-0, as the rotations of the flux need it:
+// the product with +-1 is exact, so one FMA rounds like the two products and the sum
+// (signs of zeros included) at a third of the operations
+__device__ __forceinline__ double rot(double a, double c, double b, double d) {
+  return (c == 1.0 || c == -1.0) ? fma(b, d, c == 1.0 ? a : -a) : fma(a, c, d == 1.0 ? b : -b);
 }
 
 // flux through a face of unit normal (nx, ny): rotate, x-flux, rotate back
-// (src/Flux.c:126-172).  The products with 0 and +-1 are kept: they fix the
+// (src/Flux.c:126-172).  The products with 0 are kept (in FMAs): they fix the
 // signs of zeros exactly as the reference computes them.
-__device__ __forceinline__ void flux_normal(const double (&U)[NV], double (&F)[NV], double nx,
-                                            double ny) {
-  const double tx = ny, ty = -nx;
+template <int DIR>
+__device__ __forceinline__ void flux_normal(const double (&U)[NV], double (&F)[NV]) {
+  constexpr double nx = DIR == 1 ? 1.0 : 0.0, ny = DIR == 1 ? 0.0 : 1.0;
+  constexpr double tx = ny, ty = -nx;
   double W[NV], G[NV], a, b;
   W[0] = U[0];
-  W[1] = U[1] * nx + U[2] * ny;
-  W[2] = U[1] * tx + U[2] * ty;
+  W[1] = rot(U[1], nx, U[2], ny);
+  W[2] = rot(U[1], tx, U[2], ty);
   W[3] = U[3];
-  a = U[4] * nx + U[5] * ny;
-  b = U[5] * nx + U[6] * ny;
-  W[4] = a * nx + b * ny;
-  W[5] = a * tx + b * ty;
-  a = U[4] * tx + U[5] * ty;
-  b = U[5] * tx + U[6] * ty;
-  W[6] = a * tx + b * ty;
-  W[7] = U[7] * nx + U[8] * ny;
-  W[8] = U[7] * tx + U[8] * ty;
+  a = rot(U[4], nx, U[5], ny);
+  b = rot(U[5], nx, U[6], ny);
+  W[4] = rot(a, nx, b, ny);
+  W[5] = rot(a, tx, b, ty);
+  a = rot(U[4], tx, U[5], ty);
+  b = rot(U[5], tx, U[6], ty);
+  W[6] = rot(a, tx, b, ty);
+  W[7] = rot(U[7], nx, U[8], ny);
+  W[8] = rot(U[7], tx, U[8], ty);
   grad13_flux_x(W, G);
   F[0] = G[0];
-  F[1] = G[1] * nx + G[2] * tx;
-  F[2] = G[1] * ny + G[2] * ty;
+  F[1] = rot(G[1], nx, G[2], tx);
+  F[2] = rot(G[1], ny, G[2], ty);
   F[3] = G[3];
-  a = G[4] * nx + G[5] * tx;
-  b = G[5] * nx + G[6] * tx;
-  F[4] = a * nx + b * tx;
-  F[5] = a * ny + b * ty;
-  a = G[4] * ny + G[5] * ty;
-  b = G[5] * ny + G[6] * ty;
-  F[6] = a * ny + b * ty;
-  F[7] = G[7] * nx + G[8] * tx;
-  F[8] = G[7] * ny + G[8] * ty;
+  a = rot(G[4], nx, G[5], tx);
+  b = rot(G[5], nx, G[6], tx);
+  F[4] = rot(a, nx, b, tx);
+  F[5] = rot(a, ny, b, ty);
+  a = rot(G[4], ny, G[5], ty);
+  b = rot(G[5], ny, G[6], ty);
+  F[6] = rot(a, ny, b, ty);
+  F[7] = rot(G[7], nx, G[8], tx);
+  F[8] = rot(G[7], ny, G[8], ty);
 }
+#endif
 
+#if MBM_FAST_ARITH
 // damping factor of the direct production integration (src/Flux.c:213-223)
 template <int FLAG>
 __device__ __forceinline__ double rdamp(double z) {
   if (FLAG == -1 || FLAG == 0) return fdiv(1 + 0.5 * z - 0.25 * z * z, 1 + z + 0.25 * z * z);
   if (FLAG == 1) return fdiv(1 + z, 1 + z + 0.25 * z * z);
-  if (FLAG == 2) return MBM_FAST_ARITH ? 1.0 : fdiv(1 + 0.5 * z, 1 + 0.5 * z);   // the identity
+  if (FLAG == 2) return 1.0;     // (1 + z/2) / (1 + z/2)
   return fdiv(1.0, 1 + 0.5 * z);
 }
+#else
+// Damping factors of the direct production integration (src/Flux.c:213-223) at one
+// argument: flags 0 (= -1) and 1 share a denominator, hence one reciprocal; flag 2 is
+// (1 + z/2) / (1 + z/2), which is 1 in any rounding; flag 3 is a reciprocal.  For
+// 0 <= z < 2^200 every numerator is 0 or in the range of mk_div; otherwise (NaN, a negative
+// or huge z) IEEE division.
+__device__ __forceinline__ bool damp_in(double z) { return (unsigned)__double2hiint(z) < (1223u << 20); }
+
+__device__ __forceinline__ void damp01(double z, double& r0, double& r1) {
+  const double s = 0.25 * z * z, n0 = 1 + 0.5 * z - s, n1 = 1 + z;
+  const Recip D(n1 + s);
+  r0 = mk_div(n0, D.y, D.r);
+  r1 = mk_div(n1, D.y, D.r);
+  if (__builtin_expect(D.bad || !damp_in(z), 0)) {
+    r0 = div_ieee(n0, D.y);
+    r1 = div_ieee(n1, D.y);
+  }
+}
+
+__device__ __forceinline__ void damp23(double z, double& r2, double& r3) {
+  const Recip D(1 + 0.5 * z);
+  r2 = 1.0;
+  r3 = D.r;
+  if (__builtin_expect(D.bad || !damp_in(z), 0)) {
+    r2 = div_ieee(D.y, D.y);
+    r3 = div_ieee(1.0, D.y);
+  }
+}
+#endif
 
 // The collision number z = dt nu0 rho sqrt(theta) / Kn of ProductionsDirect
 // (src/Flux.c:230-267 with CollFreq, src/Scenario.c:28-42; nu0 = 1): the same
-// expression for every flag, so one evaluation serves all of a cell's flags.  Kn is in
-// the safe range (checked when the kernel starts); the numerator's range decides
-// between the shared-reciprocal quotient and IEEE division.
+// expression for every flag, so one evaluation serves all of a cell's flags.
 __device__ __forceinline__ double coll_of(const double (&P)[NV], double dt, const Recip& Kn) {
   const double nu0 = 1.0;
-  const double num = nu0 * P[0] * fsqrt(P[3]);
-  return (__builtin_expect(mk_in(num), 1) ? Kn.exact(num) : div_ieee(num, Kn.y)) * dt;
+  return quotient(nu0 * P[0] * fsqrt(P[3]), Kn) * dt;
 }
 
 // ProductionsDirect (src/Flux.c:230-267) with ExternalForce (src/Scenario.c:28-42;
@@ -319,16 +351,18 @@ __device__ __forceinline__ void relax_d(const double (&P)[NV], double (&Out)[NV]
   moments_e(rho, v1, v2, E, T11, T12, T22, d2 * P[7], d2 * P[8], Out);
 }
 
-// ProductionsDirect of flag FLAG from the primitives P: writes the relaxed moments,
-// returns 0.5*(1 - R(2z/3))
-template <int FLAG>
-__device__ __forceinline__ double relax(const double (&P)[NV], double (&Out)[NV], double dt,
-                                        const Recip& Kn, double F) {
+// ProductionsDirect of flag -1 from the primitives P: writes the relaxed moments
+__device__ __forceinline__ void relax_m1(const double (&P)[NV], double (&Out)[NV], double dt,
+                                         const Recip& Kn, double F) {
   const double coll = coll_of(P, dt, Kn);
-  const double d1 = rdamp<FLAG>(coll);
-  const double d2 = rdamp<FLAG>(2.0 / 3 * coll);
-  relax_d<FLAG>(P, Out, dt, F, d1, d2);
-  return 0.5 * (1 - d2);
+#if MBM_FAST_ARITH
+  const double d1 = rdamp<-1>(coll), d2 = rdamp<-1>(2.0 / 3 * coll);
+#else
+  double d1, d2, unused;
+  damp01(coll, d1, unused);
+  damp01(2.0 / 3 * coll, d2, unused);
+#endif
+  relax_d<-1>(P, Out, dt, F, d1, d2);
 }
 
 #if MBM_FAST_ARITH
@@ -405,12 +439,6 @@ __device__ __forceinline__ void push_moments(const double (&U)[NV], double g, do
 // -1 only by the force acting on the velocity before the moments are formed.
 #endif
 
-// only the CFL share of relax<FLAG> (same z, same factor)
-template <int FLAG>
-__device__ __forceinline__ double relax_cfl(const double (&P)[NV], double dt, const Recip& Kn) {
-  return 0.5 * (1 - rdamp<FLAG>(2.0 / 3 * coll_of(P, dt, Kn)));
-}
-
 // Limit1 (src/Limiter.c:26-59)
 __device__ __forceinline__ double superbee_phi(double r) {
   if (r < 0.0) return 0.0;
@@ -430,6 +458,48 @@ __device__ __forceinline__ double limit(double d1, double d2) {
   const double w1 = fabs(d1) + eps, w2 = fabs(d2) + eps;
   return fdiv(w1 * d2 + w2 * d1, w1 + w2);
 }
+
+#if !MBM_FAST_ARITH
+// L = Limit1(d1, d2) and the slope L / h of the nine primitives (src/Main.c:346-349), D =
+// Recip(h), h in the safe range.  The harmonic limiter's quotient has a denominator of its
+// own, |d1| + |d2| + 2e-10: nine reciprocals without a branch, and one check of the set
+// (numerators within 2^+-400 or zero, denominators below 2^80, so that L itself is within
+// the range the division by h admits).
+template <int LIM>
+__device__ __forceinline__ void slopes(const double (&d1)[NV], const double (&d2)[NV], const Recip& D,
+                                       double (&S)[NV]) {
+  if (LIM == 0) {
+#pragma unroll
+    for (int n = 0; n < NV; n++) S[n] = 0.0;      // 0 / h
+    return;
+  }
+  double L[NV];
+  if (LIM != 4) {
+#pragma unroll
+    for (int n = 0; n < NV; n++) L[n] = limit<LIM>(d1[n], d2[n]);
+    quotients(L, D, S);
+    return;
+  }
+  const double eps = 1.0e-10;
+  MkRange g;
+  unsigned md = 0u;
+  int ones = 0;
+#pragma unroll
+  for (int n = 0; n < NV; n++) {
+    const double w1 = fabs(d1[n]) + eps, w2 = fabs(d2[n]) + eps;
+    const double x = w1 * d2[n] + w2 * d1[n], y = w1 + w2;
+    g.add(x);
+    md = max(md, (unsigned)__double2hiint(y));
+    ones |= __double2loint(y) == -1;
+    L[n] = mk_div(x, y, mk_rcp(y));
+    S[n] = mk_div(L[n], D.y, D.r);
+  }
+  if (__builtin_expect(g.lo < (623u << 21) || g.hi >= (1424u << 21) || md >= (1103u << 20) || ones || D.bad, 0)) {
+#pragma unroll
+    for (int n = 0; n < NV; n++) S[n] = div_ieee(limit<LIM>(d1[n], d2[n]), D.y);
+  }
+}
+#endif
 
 #if MBM_FAST_ARITH
 // Conservative(P) and the Grad-13 flux along x of the same state (src/Flux.c:61-119
@@ -520,37 +590,37 @@ __device__ __forceinline__ double hll(const double (&PL_)[NV], const double (&PR
 // DIR = 1: x face (normal (1,0)), DIR = 2: y face (normal (0,1)).  The
 // diffusive scale FFlux/GFlux return is 0, so lamDiff(0/(cMax*dx)) is 1 for
 // every cMax and cMax/1.0 == cMax: the division is omitted without changing a bit.
+// The left side is reduced to lamR fL and UL before the right side is formed, so that one
+// side's vectors are live at a time (alpha <= 0: the mean of the fluxes, with factor 1 in
+// place of lamR).
 template <int DIR>
 __device__ __forceinline__ double hll(const double (&PL)[NV], const double (&PR)[NV],
                                       double (&flx)[NV]) {
-  constexpr double nx = DIR == 1 ? 1.0 : 0.0, ny = DIR == 1 ? 0.0 : 1.0;
   const double cR = 2.0 * sqrt(5.0 / 3 * PR[3]);
   const double cL = 2.0 * sqrt(5.0 / 3 * PL[3]);
-  double UL[NV], UR[NV], fL[NV], fR[NV];
-  conservative(PL, UL);
-  flux_normal(UL, fL, nx, ny);
-  conservative(PR, UR);
-  flux_normal(UR, fR, nx, ny);
   const double vR = PR[DIR], vL = PL[DIR];
   const double cMax = fabs(0.5 * (vL + vR)) + rmax(cR, cL);
   const double lamL = rmin(vL - cL, 0.0);
   const double lamR = rmax(vR + cR, 0.0);
   const double alph = lamR - lamL;
-  if (alph > 0.0) {
-    Recip A(alph);
+  const bool pos = alph > 0.0;
+  double UL[NV], UR[NV], f[NV], A[NV];
+  conservative(PL, UL);
+  flux_normal<DIR>(UL, f);
+  const double kL = pos ? lamR : 1.0;
+#pragma unroll
+  for (int n = 0; n < NV; n++) A[n] = kL * f[n];
+  conservative(PR, UR);
+  flux_normal<DIR>(UR, f);
+  if (pos) {
+    const Recip D(alph);
     double num[NV];
 #pragma unroll
-    for (int n = 0; n < NV; n++) {
-      num[n] = lamR * fL[n] - lamL * fR[n] + lamL * lamR * (UR[n] - UL[n]);
-      flx[n] = A.div(num[n]);
-    }
-    if (__builtin_expect(A.bad, 0)) {
-#pragma unroll
-      for (int n = 0; n < NV; n++) flx[n] = div_ieee(num[n], alph);
-    }
+    for (int n = 0; n < NV; n++) num[n] = A[n] - lamL * f[n] + lamL * lamR * (UR[n] - UL[n]);
+    quotients(num, D, flx);
   } else {
 #pragma unroll
-    for (int n = 0; n < NV; n++) flx[n] = 0.5 * (fL[n] + fR[n]);
+    for (int n = 0; n < NV; n++) flx[n] = 0.5 * (A[n] + f[n]);
   }
   return cMax;
 }

@@ -349,13 +349,19 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
       // relaxation of Data0 for stage 2 (flag -1: flag 0 without the force) and the
       // projection (flag 2 HEUN + 1)
       const double z = coll_of(Q, dt, Kn);
-      const double d2u = rdamp<2 * HEUN>(2.0 / 3 * z);
+      double d1u, d2u, d1p, d2p;      // flags 2 HEUN and 2 HEUN + 1, at z and 2z/3
+      if (HEUN == 0) {
+        damp01(z, d1u, d1p);
+        damp01(2.0 / 3 * z, d2u, d2p);
+      } else {
+        damp23(z, d1u, d1p);
+        damp23(2.0 / 3 * z, d2u, d2p);
+      }
       if (ok && col_cell && r >= 1 && r <= nyp - 2) {
         const double c = 0.5 * (1 - d2u);
         if (c > prod) prod = c;
       }
       if (ok && col_out && r >= NG && r <= nyp - 1 - NG && r >= w.J0 && r < w.J1) {
-        const double d1u = rdamp<2 * HEUN>(z);
         const long long idx = (long long)r * pitch + C + 1;
         double R[NV];
         relax_d<2 * HEUN>(Q, R, dt, Fx, d1u, d2u);
@@ -378,7 +384,7 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
         }
 #else
         double V[NV];
-        relax_d<2 * HEUN + 1>(Q, V, dt, Fx, rdamp<2 * HEUN + 1>(z), rdamp<2 * HEUN + 1>(2.0 / 3 * z));
+        relax_d<2 * HEUN + 1>(Q, V, dt, Fx, d1p, d2p);
         primitive(V, Q);
 #endif
       }
@@ -404,20 +410,15 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
         G[n] = fma(0.5, S[n], p0);            // lower state of the next face, parked in G
       }
 #else
-      bool sbad = false;
-#pragma unroll
-      for (int n = 0; n < NV; n++) {
-        const double pm = win.P[sm2][n][lane], p0 = win.P[sm1][n][lane], pp = win.P[s0][n][lane];
-        const double L = limit<LIM>(p0 - pm, pp - p0);
-        sbad |= !mk_in(L);
-        S[n] = mk_div(L, rdy.y, rdy.r);
-      }
-      if (__builtin_expect(sbad, 0)) {
+      {
+        double d1[NV], d2[NV];
 #pragma unroll
         for (int n = 0; n < NV; n++) {
-          const double pm = win.P[sm2][n][lane], p0 = win.P[sm1][n][lane], pp = win.P[s0][n][lane];
-          S[n] = div_ieee(limit<LIM>(p0 - pm, pp - p0), rdy.y);
+          const double p0 = win.P[sm1][n][lane];
+          d1[n] = p0 - win.P[sm2][n][lane];
+          d2[n] = win.P[s0][n][lane] - p0;
         }
+        slopes<LIM>(d1, d2, rdy, S);
       }
 #pragma unroll
       for (int n = 0; n < NV; n++) {
@@ -468,22 +469,15 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
         hi[n] = __shfl_down_sync(0xffffffffu, fma(-0.5, Sx[n], P0[n]), 1);
       }
 #else
-      bool xbad = false;
-#pragma unroll
-      for (int n = 0; n < NV; n++) {
-        P0[n] = win.P[sm2][n][lane];
-        const double d1 = P0[n] - win.P[sm2][n][(lane + 31) & 31];   // left neighbour (lane 0: unused)
-        const double L = limit<LIM>(d1, __shfl_down_sync(0xffffffffu, d1, 1));
-        xbad |= !mk_in(L);
-        Sx[n] = mk_div(L, rdx.y, rdx.r);
-      }
-      if (__builtin_expect(__any_sync(0xffffffffu, xbad), 0)) {   // warp-uniform cold path
+      {
+        double d1[NV], d2[NV];
 #pragma unroll
         for (int n = 0; n < NV; n++) {
-          const double pl = __shfl_up_sync(0xffffffffu, P0[n], 1);
-          const double pr = __shfl_down_sync(0xffffffffu, P0[n], 1);
-          Sx[n] = div_ieee(limit<LIM>(P0[n] - pl, pr - P0[n]), rdx.y);
+          P0[n] = win.P[sm2][n][lane];
+          d1[n] = P0[n] - win.P[sm2][n][(lane + 31) & 31];      // left neighbour (lane 0: unused)
+          d2[n] = __shfl_down_sync(0xffffffffu, d1[n], 1);
         }
+        slopes<LIM>(d1, d2, rdx, Sx);
       }
 #pragma unroll
       for (int n = 0; n < NV; n++) {
@@ -534,7 +528,7 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
             for (int n = 0; n < NV; n++) R0[n] = U[n];
           } else {
             primitive(U, Q);
-            relax<-1>(Q, R0, dt, Kn, Fx);
+            relax_m1(Q, R0, dt, Kn, Fx);
           }
 #pragma unroll
           for (int n = 0; n < NV; n++) R[n] += R0[n];
