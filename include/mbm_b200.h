@@ -288,7 +288,8 @@ int mbm_ghost_scatter(mbm_ctx *ctx, int *on);
  * finishes and waits on the device for its results, which takes the launch gaps out
  * of the step.  Off with MBM_PDL=0 at context creation, when a stage runs as several
  * limiter groups on forked streams, and when the step graph cannot be built with it.
- * No counterpart in the reference. */
+ * A small grid's step loop is one kernel (MBM_TILES=0 at creation: never); *on then
+ * tells of its other launches.  No counterpart in the reference. */
 int mbm_dependent_launch(mbm_ctx *ctx, int *on);
 
 /* Host-only: the resolved ghost-cell sources of a block table, 4 ints per ghost
@@ -323,7 +324,7 @@ int mbm_ghost_map(const mbm_block_desc *blocks, int nblocks, int *entries, int c
  * Scratch: one file-scope device array of 320 KB (held by every GPU that loads
  * the library until the process exits): at most 64 blocks and 20,064 warp work
  * items (28-column strips x 32-row segments, e.g. 16 blocks of 1024^2); larger
- * inputs return MBM_EINVAL.  Its device address is looked up by the first call on
+ * inputs return MBM_EINVAL (smaller ones are cut into shorter segments or tiles).  Its device address is looked up by the first call on
  * each device, with that device current -- make that first call before any stream
  * capture.  Every call shares the array and clears what must start at zero; calls
  * that overlap on the GPU race.  Errors: mbm_last_error(NULL). */

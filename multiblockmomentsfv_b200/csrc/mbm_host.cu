@@ -23,11 +23,17 @@
 namespace mbm {
 namespace bitwise {
 cudaError_t launch_stage(int lim, const StageArgs& a, int grid, cudaStream_t s);
+cudaError_t launch_tiles(const StageArgs& a, cudaStream_t s);
+cudaError_t launch_tile_steps(const TileLoop& L, int grid, cudaStream_t s);
+int tile_ctas_per_sm();
 int stage_ctas_per_sm(int heun);
 int stage_cta_warps();
 }
 namespace fastmath {
 cudaError_t launch_stage(int lim, const StageArgs& a, int grid, cudaStream_t s);
+cudaError_t launch_tiles(const StageArgs& a, cudaStream_t s);
+cudaError_t launch_tile_steps(const TileLoop& L, int grid, cudaStream_t s);
+int tile_ctas_per_sm();
 int stage_ctas_per_sm(int heun);
 int stage_cta_warps();
 }
@@ -98,6 +104,7 @@ struct mbm_ctx {
   double* staging = nullptr;        // array-of-structs transfer buffer, one block
   GhostEntry* dghost = nullptr;
   int nghost = 0;
+  int* dgoff = nullptr;             // per block, its first entry of dghost
   std::vector<int> dir_off;         // [block*4+side] -> first Dirichlet row, -1 if none
   double* ddir = nullptr;
   int ndir = 0;
@@ -110,6 +117,13 @@ struct mbm_ctx {
   std::vector<GhostScatter> gs_ent;  // host: the entries in owner order
   GhostScatter* dgs = nullptr;       // per stage (gs_ent.size() apart): the entries in work-item order
   int2* dgs_item = nullptr;          // per stage (max_items apart): first entry and count of each item
+  // small grids: stages in tiles (mbm_tile.cuh), the step loop one persistent kernel of
+  // tile_grid CTAs; dwork then holds the tiles
+  bool tiles = false;
+  bool tile_loop = false;           // (no adjoint records, few tiles per CTA)
+  int tile_grid = 0;
+  unsigned* dsync = nullptr;        // tile_steps: TileLoop::sync (4 words) and ::lam behind it
+  unsigned* hsync = nullptr;        // pinned: whether one of its waits ran out
   Work* dwork = nullptr;            // the work tables of the two Heun stages, max_items apart
   long long max_items = 0;
   int nwork[2] = {0, 0};
@@ -388,7 +402,7 @@ static void build_work(mbm_ctx* c, double seg_rows, std::vector<Work>& w, std::v
 }
 
 // rebuild the work table for segments of `seg` rows; the table lives in the same
-// device buffer (sized for 8-row segments)
+// device buffer (sized for 2-row segments)
 // work items of a segment length (host only; the count build_work makes)
 static long long count_items(const mbm_ctx* c, double seg_rows) {
   long long n = 0;
@@ -456,6 +470,37 @@ static int set_segments(mbm_ctx* c, double seg, int h = -1) {
   return MBM_OK;
 }
 
+// what every launch of a stage is given: the context's tables and layers (or the caller's)
+static StageArgs stage_args(mbm_ctx* c, int heun, double* const* bufs) {
+  StageArgs a{};
+  a.blk = c->dblk;
+  a.cases = c->dcase;
+  for (int l = 0; l < 3; l++) a.buf[l] = bufs ? bufs[l] : c->buf[l];
+  a.lam = c->dlam;
+  a.heun = heun;
+  a.rlx = c->rlx;
+  return a;
+}
+
+static size_t tile_scratch(const mbm_ctx* c) { return sizeof(unsigned) * 4 + sizeof(unsigned long long) * 18 * c->nblk; }
+
+// the tiles of every block: 28 columns x TILE_ROWS rows over the face range, as build_work's
+// strips and segments
+static int set_tiles(mbm_ctx* c) {
+  std::vector<Work> w;
+  for (int b = 0; b < c->nblk; b++)
+    for (int J0 = 1; J0 <= c->hblk[b].nyp - 3; J0 += TILE_ROWS)
+      for (int I0 = 1; I0 <= c->hblk[b].nxp - 3; I0 += STRIP) w.push_back(Work{b, I0, J0, J0 + TILE_ROWS});
+  for (int h = 0; h < 2; h++) {
+    c->nwork[h] = (int)w.size();
+    c->seg_rows[h] = TILE_ROWS;
+    c->groups[h].assign(1, LimGroup{0, 0, (int)w.size(), {c->tile_grid, c->tile_grid}});
+  }
+  CK(cudaMemcpyAsync(c->dwork, w.data(), sizeof(Work) * w.size(), cudaMemcpyHostToDevice, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  return MBM_OK;
+}
+
 // one Heun stage of every block: one persistent launch per limiter group
 // (with several limiter groups, group k > 0 runs on aux stream k-1, so that one
 // group's CTAs fill the SMs another group's tail leaves idle).  rlx_read (stage 2):
@@ -464,6 +509,14 @@ static int set_segments(mbm_ctx* c, double seg, int h = -1) {
 // Data0 just before.
 static cudaError_t launch_stages(mbm_ctx* c, int heun, int sel_in, int sel_d0, int sel_out, int rlx_read,
                                  double* const* bufs = nullptr, bool fill = false) {
+  if (c->tiles) {
+    StageArgs a = stage_args(c, heun, bufs);
+    a.work = c->dwork;
+    a.nwork = c->nwork[heun];
+    a.sel_in = sel_in; a.sel_d0 = sel_d0; a.sel_out = sel_out;
+    a.rlx_read = heun == 1 && rlx_read;
+    return c->fast ? fastmath::launch_tiles(a, c->stream) : bitwise::launch_tiles(a, c->stream);
+  }
   const std::vector<LimGroup>& groups = c->groups[heun];
   const int ng = (int)groups.size();
   cudaError_t e0;
@@ -475,17 +528,11 @@ static cudaError_t launch_stages(mbm_ctx* c, int heun, int sel_in, int sel_d0, i
   for (int k = 0; k < ng; k++) {
     const LimGroup& g = groups[k];
     cudaStream_t st = k == 0 ? c->stream : c->aux[k - 1];
-    StageArgs a{};
-    a.blk = c->dblk;
+    StageArgs a = stage_args(c, heun, bufs);
     a.work = c->dwork + heun * c->max_items + g.start;
     a.nwork = g.count;
-    a.cases = c->dcase;
-    for (int l = 0; l < 3; l++) a.buf[l] = bufs ? bufs[l] : c->buf[l];
-    a.lam = c->dlam;
     a.queue = c->dqueue + heun * 5 + g.lim;
     a.sel_in = sel_in; a.sel_d0 = sel_d0; a.sel_out = sel_out;
-    a.heun = heun;
-    a.rlx = c->rlx;
     a.rlx_read = heun == 1 && rlx_read;
     // bulk tensor copies: fast stage 2 on the context's own layers (the maps cover TMP
     // and rlx; the adjoint's recomputation passes other buffers and keeps cp.async)
@@ -544,7 +591,9 @@ static int push_cases(mbm_ctx* c) {
 // it times each Heun stage for each candidate on a uniform state at rest and keeps,
 // per stage, the fastest (the two stages have their own work tables: at 4 x 1024^2
 // stage 1 ran best at 24 rows, stage 2 at 29); the choice is cached per (strip rows,
-// blocks, limiter mix, CTAs/SM) for the life of the process.
+// blocks, limiter mix, CTAs/SM) for the life of the process.  Lengths down to 2 rows: where
+// few warps are resident, a warp's march is the time, 4 rows of warm-up or not (a step of
+// 4 x 128^2 cells: 116 us bitwise and 54 us fast with 8 rows at the least, 75 and 43 with 2).
 static std::mutex g_tune_mu;
 static std::map<std::tuple<long long, int, int, int>, std::array<double, 2>> g_tune_cache;
 
@@ -609,13 +658,14 @@ static int autotune(mbm_ctx* c) {
   // (6,956 items, 3.92 waves) 3 % faster than 24, 20 rows 5 % slower, 21.4 rows (7,104
   // items, 4 waves) 1.7 % faster than 22.
   std::vector<double> cand;
+  for (int seg = 2; seg < 8; seg++) cand.push_back(seg);
   for (int seg = 8; seg <= 64; seg += 2) cand.push_back(seg);
   for (int h = 0; h < 2; h++) {              // the resident warps of each stage
     if (h == 1 && c->ctas_per_sm[1] == c->ctas_per_sm[0]) break;
     const long long W = (long long)c->nsm * c->ctas_per_sm[h] * c->cta_warps;
-    const long long most = count_items(c, 8.0), least = count_items(c, 64.0);
+    const long long most = count_items(c, 2.0), least = count_items(c, 64.0);
     for (long long k = (least + W - 1) / W; k * W < most && k <= 64; k++) {
-      double lo = 8.0, hi = 64.0;              // count_items(hi) <= k W < count_items(lo)
+      double lo = 2.0, hi = 64.0;              // count_items(hi) <= k W < count_items(lo)
       for (int it = 0; it < 40; it++) {
         const double mid = 0.5 * (lo + hi);
         if (count_items(c, mid) <= k * W) hi = mid;
@@ -771,6 +821,15 @@ extern "C" int mbm_create_batch(const mbm_block_desc* blocks, int nblocks, const
 
 // the context proper, from a block table whose ghost map is resolved; shard: the
 // exchange plan of a case split over ranks (nullptr otherwise)
+// whether a grid of this many tiles is advanced in tiles (MBM_TILES=1: any grid, 0: none)
+static bool tiles_pay(const mbm_ctx* c, long long tiles) {
+  const char* env = getenv("MBM_TILES");
+  if (env) return atoi(env) != 0;
+  bool one = true;
+  for (int k = 1; k < c->ncase; k++) one = one && c->hcase[k].limiter == c->hcase[0].limiter;
+  return tiles <= (c->fast ? TILE_MOST_FAST : one ? TILE_MOST_EXACT : TILE_MOST_EXACT_BATCH);
+}
+
 static int create_impl(const std::vector<mbm_block_desc>& glob, const std::vector<int>& blk_case,
                        const mbm_case_desc* cases, int ncases, const mbm_params* params,
                        const std::vector<Resolved>& res, const std::vector<int>& dir_off, int ndir,
@@ -872,6 +931,14 @@ static int create_impl(const std::vector<mbm_block_desc>& glob, const std::vecto
     gm[i] = e;
   }
   c->nghost = (int)gm.size();
+  // the map lists the ghost cells block by block, row by row
+  std::vector<int> goff(nblocks);
+  for (int b = 0, off = 0; b < nblocks; b++) {
+    goff[b] = off;
+    off += c->hblk[b].nxp * c->hblk[b].nyp - glob[b].nx * glob[b].ny;
+  }
+  CKC(cudaMalloc(&c->dgoff, sizeof(int) * nblocks));
+  CKC(cudaMemcpyAsync(c->dgoff, goff.data(), sizeof(int) * nblocks, cudaMemcpyHostToDevice, c->stream));
   CKC(cudaMalloc(&c->dghost, sizeof(GhostEntry) * std::max<size_t>(1, gm.size())));
   if (!gm.empty())
     CKC(cudaMemcpyAsync(c->dghost, gm.data(), sizeof(GhostEntry) * gm.size(), cudaMemcpyHostToDevice, c->stream));
@@ -956,7 +1023,20 @@ static int create_impl(const std::vector<mbm_block_desc>& glob, const std::vecto
     c->ctas_per_sm[hh] = c->fast ? fastmath::stage_ctas_per_sm(hh) : bitwise::stage_ctas_per_sm(hh);
   c->cta_warps = c->fast ? fastmath::stage_cta_warps() : bitwise::stage_cta_warps();
   long long max_items = 0;
-  for (auto& d : c->hblk) max_items += (long long)((d.nxp - 3 + STRIP - 1) / STRIP) * ((d.nyp - 3 + 7) / 8 + 1);
+  for (auto& d : c->hblk) max_items += (long long)((d.nxp - 3 + STRIP - 1) / STRIP) * ((d.nyp - 3 + 1) / 2 + 1);
+  const int tile_ctas = c->fast ? fastmath::tile_ctas_per_sm() : bitwise::tile_ctas_per_sm();
+  long long tiles = 0;
+  for (auto& d : c->hblk)
+    tiles += (long long)((d.nxp - 3 + STRIP - 1) / STRIP) * ((d.nyp - 3 + TILE_ROWS - 1) / TILE_ROWS);
+  c->tiles = params->segment_rows <= 0 && !c->gscatter && !c->dtmap && tile_ctas > 0 && tiles_pay(c, tiles);
+  if (c->tiles) {
+    max_items = (tiles + 1) / 2;
+    c->tile_grid = (int)std::min<long long>(tiles, (long long)c->nsm * tile_ctas);
+    c->tile_loop = !c->adjoint && !shard && tiles <= (long long)TILE_MAX * c->tile_grid;
+    CKC(cudaMalloc(&c->dsync, tile_scratch(c)));
+    CKC(cudaMallocHost(&c->hsync, sizeof(unsigned)));
+    *c->hsync = 0;
+  }
   c->max_items = std::max<long long>(1, max_items);
   CKC(cudaMalloc(&c->dwork, sizeof(Work) * 2 * c->max_items));
   if (c->gscatter) {
@@ -964,7 +1044,8 @@ static int create_impl(const std::vector<mbm_block_desc>& glob, const std::vecto
     CKC(cudaMalloc(&c->dgs_item, sizeof(int2) * 2 * c->max_items));
   }
   {
-    int st0 = params->segment_rows > 0 ? set_segments(c, std::max(8, params->segment_rows)) : autotune(c);
+    int st0 = params->segment_rows > 0 ? set_segments(c, std::max(8, params->segment_rows))
+              : c->tiles ? set_tiles(c) : autotune(c);
     if (st0) return bail(st0);
   }
 
@@ -997,10 +1078,13 @@ static int create_impl(const std::vector<mbm_block_desc>& glob, const std::vecto
     return MBM_OK;
   }
 
-  // the step loop: while (any case live) { stage 1; fill TMP; stage 2; fill NEW; control }
   {
     const char* pe = getenv("MBM_PDL");
     c->pdl = !(pe && atoi(pe) == 0);
+  }
+  // the step loop: while (any case live) { stage 1; fill TMP; stage 2; fill NEW; control }
+  // (in tiles without checkpoints: tile_steps)
+  if (!c->tile_loop) {
     auto build_graph = [&]() -> cudaError_t {
       cudaError_t e;
       cudaGraphConditionalHandle h;
@@ -1067,10 +1151,13 @@ extern "C" int mbm_destroy(mbm_ctx* c) {
   cudaFree(c->staging);
   cudaFree(c->dblk);
   cudaFree(c->dghost);
+  cudaFree(c->dgoff);
   cudaFree(c->ddir);
   cudaFree(c->dgs);
   cudaFree(c->dgs_item);
   cudaFree(c->dwork);
+  cudaFree(c->dsync);
+  if (c->hsync) cudaFreeHost(c->hsync);
   cudaFree(c->dcase);
   if (c->hcase) cudaFreeHost(c->hcase);
   cudaFree(c->dlam);
@@ -1316,7 +1403,26 @@ extern "C" int mbm_steps_batch_async(mbm_ctx* c, const double* t, const double* 
   }
   int st = push_cases(c);
   if (st) return st;
-  if (any && !c->host_loop) {
+  if (any && !c->host_loop && c->tile_loop) {
+    TileLoop L{};
+    L.st = stage_args(c, 0, nullptr);
+    L.st.work = c->dwork;
+    L.st.nwork = c->nwork[0];
+    L.st.rlx_read = 1;
+    L.st.dirichlet = c->ddir;
+    L.st.ghosts = c->dghost;
+    L.st.goff = c->dgoff;
+    L.ncase = c->ncase;
+    L.nghost = c->nghost;
+    L.nblk = c->nblk;
+    L.trace = c->dtrace;
+    L.sync = c->dsync;
+    L.lam = (unsigned long long*)(c->dsync + 4);
+    CK(cudaMemsetAsync(c->dsync, 0, tile_scratch(c), c->stream));
+    CK(c->fast ? fastmath::launch_tile_steps(L, c->tile_grid, c->stream)
+               : bitwise::launch_tile_steps(L, c->tile_grid, c->stream));
+    CK(cudaMemcpyAsync(c->hsync, c->dsync + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+  } else if (any && !c->host_loop) {
     CK(cudaMemsetAsync(c->dqueue, 0, sizeof(int) * 10, c->stream));
     CK(cudaGraphLaunch(c->gexec, c->stream));
   } else if (any) {
@@ -1342,6 +1448,7 @@ extern "C" int mbm_steps_batch_wait(mbm_ctx* c, double* t, int* nsteps, int* nre
   int st;
   CK(cudaMemcpyAsync(c->hcase, c->dcase, sizeof(CaseDev) * c->ncase, cudaMemcpyDeviceToHost, c->stream));
   if ((st = wait_stream(c))) return st;
+  if (c->hsync && *c->hsync) return fail(c, MBM_ETIMEOUT, "a bounded wait of the step loop's grid barrier ran out");
   int worst = 0;
   for (int k = 0; k < c->ncase; k++) {
     const CaseDev& h = c->hcase[k];

@@ -22,6 +22,14 @@ namespace mbm {
 constexpr int NV = 9;           // moments per cell (src/defs.h:11)
 constexpr int NG = 3;           // ghost layers per edge (src/defs.h:14)
 constexpr int STRIP = 28;        // output columns per warp strip (32 lanes - 2 - 2 halo)
+constexpr int TILE_ROWS = 4;     // output rows of a tile (28 x 4 cells, mbm_tile.cuh)
+// The most tiles of a grid that is advanced in tiles rather than by the row march: where the
+// two measured alike (a step of 4 x n^2 cells, harmonic, tiles / march in us):
+//   bitwise  n = 61: 23.6 / 51.3   192: 92 / 103   224 (2,052 tiles): 128 / 146   240: 144 / 145
+//   fast     n = 61: 14.6 / 33.3   192: 49 / 53    224: 68 / 68   256 (2,600 tiles): 97 / 78
+// Several limiters in a batch are as many launches for the march, none more for the tiles
+// (bitwise, 8 cases, 4,668 tiles: 318 / 359; 7,469: 482 / 488; fast, 2,567: 98 / 92).
+constexpr int TILE_MOST_EXACT = 2100, TILE_MOST_EXACT_BATCH = 7000, TILE_MOST_FAST = 1700;
 constexpr int CTA_WARPS = 4;     // warps per CTA of the persistent stage kernel
 constexpr int MAX_TRACE = 4096;  // progress records kept per case and Steps call
 
@@ -115,6 +123,18 @@ struct StageArgs {
   // CTA 0 consumes it (sets it to 0) and withholds its first bulk copy, so that its
   // bounded wait runs out -- one launch, also when the launch is replayed from a graph
   int* tma_drop;
+  const GhostEntry* ghosts;  // tile_steps: the resolved ghost map
+  const int* goff;           // and per block its first entry in it
+};
+
+constexpr int TILE_MAX = 26;    // tiles a CTA of tile_steps may keep
+
+struct TileLoop {      // the step loop of tile_steps (mbm_tile.cuh)
+  StageArgs st;
+  int ncase, nghost, nblk;
+  double* trace;
+  unsigned long long* lam;   // three sets of the blocks' maxima
+  unsigned* sync;            // [0] arrivals at the grid barrier, [2] a wait ran out, [3] cases done
 };
 
 constexpr int TMAP_BYTES = 128;   // sizeof(CUtensorMap)

@@ -1,6 +1,6 @@
 // mbm_kernels.cu -- the ghost-cell gather, the step controller, checkpoints,
 // output staging and the layout transposes, and the bitwise instantiation of the
-// Heun stage kernel (mbm_stage.cuh).
+// Heun stage kernels (mbm_stage.cuh, mbm_tile.cuh).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -9,7 +9,7 @@
 // CTAs per SM (238 / 226 registers, no spills) run a 4 x 1024^2 step in 1.96 ms, three (168,
 // spilling 40-64 bytes) in 2.01 ms, and 4 x 256^2 in 0.196 against 0.232 ms
 #define STAGE_MIN_CTAS 2
-#include "mbm_stage.cuh"   // the stage kernel in namespace mbm::bitwise
+#include "mbm_tile.cuh"    // the stage kernels in namespace mbm::bitwise
 
 namespace mbm {
 
@@ -18,9 +18,7 @@ thread_local bool tl_pdl = false;
 using namespace bitwise;    // the output conversion uses the bitwise Primitive
 
 // ---------------------------------------------------------------- ghost fill --
-// SetBoundary (src/Boundary.c:173-193) as a gather: the host resolved the two
-// sweeps into the final source of every ghost cell (an interior cell of some
-// block, with the composed wall signs of src/Scenario.c:57-63, or a Dirichlet row).
+// SetBoundary as a gather, one thread per ghost cell (ghost_fill, mbm_step.cuh)
 __global__ void ghost_kernel(const BlockDev* __restrict__ blk, const CaseDev* __restrict__ cases,
                              const GhostEntry* __restrict__ map, int n, double* buf0,
                              double* buf1, double* buf2, const double* __restrict__ dirichlet,
@@ -29,96 +27,20 @@ __global__ void ghost_kernel(const BlockDev* __restrict__ blk, const CaseDev* __
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const GhostEntry e = map[i];
-  const BlockDev D = blk[e.dst_blk];
-  const CaseDev& cs = cases[D.case_id];
+  const CaseDev& cs = cases[blk[e.dst_blk].case_id];
   if (cs.done) return;
   const int l = phys_layer(sel, cs.cur);
-  double* layer = l == 0 ? buf0 : (l == 1 ? buf1 : buf2);
-  double* dst = layer + D.off + e.dst;
-  const int sblk = e.src_blk_flags & 0xffff;
-  const bool fx = (e.src_blk_flags >> 16) & 1, fy = (e.src_blk_flags >> 17) & 1;
-#pragma unroll
-  for (int m = 0; m < NV; m++) {
-    double v;
-    if (e.src_blk_flags & GHOST_REMOTE) {          // a source cell on another rank
-      v = recv[(size_t)e.src * NV + m];
-    } else if (e.src >= 0) {
-      const BlockDev S = blk[sblk];
-      v = layer[S.off + m * S.plane + e.src];
-    } else {
-      v = dirichlet[(size_t)(-(e.src + 1)) * NV + m];
-    }
-    const bool flip = (fx && (m == 1 || m == 5 || m == 7)) != (fy && (m == 2 || m == 5 || m == 8));
-    dst[m * D.plane] = flip ? -v : v;
-  }
+  ghost_fill(blk, e, l == 0 ? buf0 : (l == 1 ? buf1 : buf2), dirichlet, recv);
 }
 
 // ---------------------------------------------------------------- controller --
-// One Steps iteration's bookkeeping for every case (src/Main.c:196-216, 253-283):
-// CFL = max over stages and blocks of dt*lx/dx + dt*ly/dy + prod; reject if
-// CFL > CFLmax, else accept, swap DATA/NEW and advance t; next dt = dt*CFLreg/CFL.
+// one Steps iteration's bookkeeping (control_cases, mbm_step.cuh)
 __global__ void control_kernel(CaseDev* cases, int ncases, const BlockDev* __restrict__ blk,
                                unsigned long long* lam, double* trace, int* queues,
                                cudaGraphConditionalHandle h, int use_handle, const double* cfl_ext) {
   pdl_enter();
   if (threadIdx.x < 10) queues[threadIdx.x] = 0;  // work counters [stage][limiter]
-  int live = 0;
-  for (int c = threadIdx.x; c < ncases; c += blockDim.x) {
-    CaseDev& cs = cases[c];
-    if (cs.done) continue;
-    const double dt = cs.dt;
-    double cfl1 = 0.0, cfl2 = 0.0;
-    for (int b = cs.blk0; b < cs.blk0 + cs.nblk; b++) {
-      unsigned long long* s = lam + (size_t)b * 6;
-      const double dx = blk[b].dx, dy = blk[b].dy;
-      const double v1 = dt * __longlong_as_double(s[0]) / dx + dt * __longlong_as_double(s[1]) / dy +
-                        __longlong_as_double(s[2]);
-      const double v2 = dt * __longlong_as_double(s[3]) / dx + dt * __longlong_as_double(s[4]) / dy +
-                        __longlong_as_double(s[5]);
-      if (v1 > cfl1) cfl1 = v1;
-      if (v2 > cfl2) cfl2 = v2;
-      for (int k = 0; k < 6; k++) s[k] = 0ull;
-    }
-    // a case split over ranks brings the max over all ranks (single-case contexts)
-    const double cfl = cfl_ext ? *cfl_ext : rmax(cfl1, rmax(cfl2, 0.0));
-    cs.cfl_last = cfl;
-    cs.attempts++;
-    cs.accepted = 0;
-    if (cs.nonfinite) {       // a stage wrote a NaN or infinity: stop before accepting it
-      // bit 2: a bounded wait for a bulk copy ran out (MBM_ETIMEOUT), else MBM_ENONFINITE
-      cs.status = (cs.nonfinite & 2) ? 3 : 2;
-      cs.done = 1;
-    } else if (cfl > cs.CFLmax) {
-      cs.dt = dt * cs.CFLreg / cfl;
-      cs.nrej++;
-    } else {
-      cs.t += dt;
-      double nd = dt * cs.CFLreg / cfl;
-      if (cs.t + nd > cs.tend) nd = cs.tend - cs.t;
-      cs.dt = nd;
-      cs.nstep++;
-      cs.cur = 1 - cs.cur;
-      cs.accepted = 1;
-      if (cs.dtlog && cs.nstep <= cs.dtlog_cap) cs.dtlog[cs.nstep - 1] = dt;   // frozen for the adjoint
-      if (cs.show_every > 0 && cs.nstep % cs.show_every == 0 && cs.trace_n < MAX_TRACE) {
-        double* r = trace + ((size_t)c * MAX_TRACE + cs.trace_n) * 4;
-        r[0] = cs.nstep; r[1] = cfl; r[2] = cs.t; r[3] = cs.dt;
-        cs.trace_n++;
-      }
-      if (!(cs.t < cs.tend) || (cs.step_cap > 0 && cs.nstep >= cs.step_cap)) cs.done = 1;
-    }
-    if (!cs.done) {
-      if (!isfinite(cfl) || !isfinite(cs.dt) || !(cs.dt > 0.0)) {
-        cs.status = 2;  // MBM_ENONFINITE
-        cs.done = 1;
-      } else if (cs.attempts >= cs.max_attempts) {
-        cs.status = 5;  // MBM_ESTEPLIMIT
-        cs.done = 1;
-      }
-    }
-    if (!cs.done) live = 1;
-  }
-  live = __syncthreads_or(live);
+  const int live = control_cases(cases, ncases, blk, lam, trace, cfl_ext);
   if (use_handle && threadIdx.x == 0) cudaGraphSetConditional(h, live ? 1u : 0u);
 }
 

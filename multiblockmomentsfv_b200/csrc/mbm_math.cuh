@@ -23,6 +23,7 @@
 #define MBM_HD __host__ __device__ __forceinline__
 #include "mbm_adjoint_math.cuh"   // primitive-form Conservative and Grad-13 flux
 #endif
+#include "mbm_div.cuh"
 #include "mbm_newton.cuh"
 
 namespace mbm {
@@ -33,40 +34,13 @@ __device__ __forceinline__ double rmax(double a, double b) { return a > b ? a : 
 __device__ __forceinline__ double rmin(double a, double b) { return a < b ? a : b; }
 __device__ __forceinline__ double rsgn(double a) { return a == 0 ? 0.0 : (a < 0 ? -1.0 : 1.0); }
 
-// ---------------------------------------------------------------------------
-// Correctly rounded division from a shared reciprocal.
-//
-// Markstein's correction step (P. Markstein, "Computation of elementary functions
-// on the IBM RISC System/6000 processor", IBM J. Res. Develop. 34(1):111-119, 1990;
-// J.-M. Muller et al., Handbook of Floating-Point Arithmetic, 2nd ed., 2018, ch. 4):
-// with r = RN(1/y) and q = RN(x*r), the remainder q*y - x is exact in one FMA and
-// RN(q - (q*y - x)*r) = RN(x/y), provided x, y and the quotient stay in the normal
-// range.  One reciprocal then serves every quotient with the same denominator at
-// three FP64 operations each, with the same bits as IEEE x/y.  For y > 0 the negated
-// remainder gives zeros their sign too: x = +-0 leaves q = +-0, the remainder q*y - x is
-// +0, and -(+0)*r + q = q.  The reciprocal is Markstein's as well: the hardware
-// approximation refined to within one unit in the last place (the third-order step of
-// mbm_newton.cuh), then RN(r + r(1 - y r)), which is RN(1/y) unless y's significand is
-// all ones (set apart).
-//
-// The hot path has no branch per quotient.  A set of quotients is checked together by
-// integer minima and maxima of its numerators' high words (MkRange: about four integer
-// instructions each, zeros admitted); a set with a numerator out of range, or whose
-// denominator is not positive or out of range, is divided by IEEE division, out of line.
-// Measured (bitwise step): 4 x 1024^2 cells, harmonic, 3.15 ms with a full test and a
-// signed-zero select per quotient (ten integer instructions) and IEEE divisions in the
-// limiter, 1.81 ms like this; 28 blocks of 30 x 10 in a stream, most sets holding a zero,
-// 143 against 129 us (checking exponents alone and sorting the zeros out in a second look:
-// 1.96 ms and 143 us).
-// Checked against x/y on the host for random and near-tie operands
-// (tests/test_division.py, tests/test_exact_division.py) and by every bitwise parity test.
+// Reciprocal, square root and lone quotients.  Bitwise: the exact division of mbm_div.cuh,
+// IEEE division and sqrt.
 //
 // Fast arithmetic (MBM_FAST_ARITH, MBM_MODE_FAST): the quotient is RN(x*r) without
-// the correction, within one unit in the last place of x/y, and nothing is checked; the
-// file is then compiled with multiply-add contraction.
-__device__ __noinline__ double div_ieee(double x, double y) { return x / y; }
-
-// Reciprocal, square root and lone quotients.  Bitwise: IEEE division and sqrt.
+// the correction, within one unit in the last place of x/y, and nothing is checked.  Its
+// multiply-adds are written out, not left to the compiler's contraction, so that every
+// kernel that evaluates these functions (row march, tiles) gets the same bits.
 // Fast arithmetic: the refined hardware approximations of mbm_newton.cuh.
 #if MBM_FAST_ARITH
 using mbm_newton::frcp;
@@ -75,48 +49,6 @@ __device__ __forceinline__ double fdiv(double x, double y) { return x * frcp(y);
 #else
 __device__ __forceinline__ double fdiv(double x, double y) { return x / y; }
 __device__ __forceinline__ double fsqrt(double x) { return sqrt(x); }
-
-constexpr unsigned MK_LO = 543u << 21;             // 2^-480, as (high word << 1)
-constexpr unsigned MK_SPAN = (961u << 21) - 1u;    // up to 2^481, exclusive
-
-// The numerators of a set: in range if each is zero or has its exponent in the admitted
-// range.  (high word << 1) - 1 + (low word != 0) is all ones for a zero and keeps the
-// order of everything else, deep subnormals included, so its minimum finds the small ones.
-struct MkRange {
-  unsigned lo = ~0u, hi = 0u;
-  __device__ __forceinline__ void add(double x) {
-    const unsigned h = 2u * (unsigned)__double2hiint(x);
-    unsigned u;
-    asm("{\n .reg .u32 t;\n add.cc.u32 t, %1, 0xffffffff;\n addc.u32 %0, %2, 0xffffffff;\n}"
-        : "=r"(u) : "r"(__double2loint(x)), "r"(h));
-    lo = min(lo, u);
-    hi = max(hi, h);
-  }
-  __device__ __forceinline__ bool bad() const { return lo < MK_LO || hi > MK_LO + MK_SPAN; }
-};
-
-__device__ __forceinline__ double mk_div(double x, double y, double r) {   // y > 0
-  const double q = x * r;
-  return fma(-fma(q, y, -x), r, q);
-}
-
-// RN(1/y) for y in range, unless y's significand is all ones
-__device__ __forceinline__ double mk_rcp(double y) {
-  const double r = mbm_newton::frcp(y);
-  return fma(fma(-y, r, 1.0), r, r);
-}
-// a significand of all ones, y = 2^k (2 - 2^-52): then RN(1/y) = 2^(-k-1) (1 + 2^-52).
-// Densities one rounding below 1 make this an everyday value of a stream at rho = 1.
-__device__ __forceinline__ double mk_rcp_all(double y) {
-  const int h = __double2hiint(y);
-  const double r = mk_rcp(y);
-  return ((h | (int)0xfff00000) & __double2loint(y)) == -1
-             ? __hiloint2double((2045 << 20) - (h & 0x7ff00000), 1) : r;
-}
-// y not positive or out of range
-__device__ __forceinline__ bool mk_bad_den(double y) {
-  return (unsigned)__double2hiint(y) - (543u << 20) >= (961u << 20);
-}
 #endif
 
 struct Recip {        // 1/y for a denominator shared by several quotients
@@ -158,6 +90,20 @@ __device__ __forceinline__ double quotient(double x, const Recip& D) {
   return q[0];
 }
 
+#if MBM_FAST_ARITH
+// Primitive (src/Flux.c:30-56)
+__device__ __forceinline__ void primitive(const double (&U)[NV], double (&P)[NV]) {
+  const double rho = U[0], r = frcp(rho), E = U[3];
+  const double v1 = U[1] * r, v2 = U[2] * r;
+  const double a = v1 * v1, b = v2 * v2;
+  const double T11 = fma(U[4], r, -a), T12 = fma(U[5], r, -(v1 * v2)), T22 = fma(U[6], r, -b);
+  P[0] = rho; P[1] = v1; P[2] = v2;
+  P[3] = fma(2 * E, r, -(a + b)) * (1.0 / 3);
+  P[4] = T11; P[5] = T12; P[6] = T22;
+  P[7] = fma(-rho, fma(T11, v1, T12 * v2), fma(-E, v1, U[7]));
+  P[8] = fma(-rho, fma(T12, v1, T22 * v2), fma(-E, v2, U[8]));
+}
+#else
 // Primitive (src/Flux.c:30-56)
 __device__ __forceinline__ void primitive(const double (&U)[NV], double (&P)[NV]) {
   const double rho = U[0];
@@ -177,7 +123,9 @@ __device__ __forceinline__ void primitive(const double (&U)[NV], double (&P)[NV]
   P[7] = U[7] - E * v1 - rho * (T11 * v1 + T12 * v2);
   P[8] = U[8] - E * v2 - rho * (T12 * v1 + T22 * v2);
 }
+#endif
 
+#if !MBM_FAST_ARITH
 // moments with an explicit energy (src/Flux.c:65-73, 255-263)
 __device__ __forceinline__ void moments_e(double rho, double v1, double v2, double E, double T11,
                                           double T12, double T22, double q1, double q2,
@@ -200,7 +148,6 @@ __device__ __forceinline__ void conservative(const double (&P)[NV], double (&U)[
   moments_e(P[0], P[1], P[2], E, P[4], P[5], P[6], P[7], P[8], U);
 }
 
-#if !MBM_FAST_ARITH
 // Grad-13 flux along x of a moment vector (src/Flux.c:79-119)
 __device__ __forceinline__ void grad13_flux_x(const double (&U)[NV], double (&F)[NV]) {
   const double rho = U[0];
@@ -281,16 +228,7 @@ __device__ __forceinline__ void flux_normal(const double (&U)[NV], double (&F)[N
 }
 #endif
 
-#if MBM_FAST_ARITH
-// damping factor of the direct production integration (src/Flux.c:213-223)
-template <int FLAG>
-__device__ __forceinline__ double rdamp(double z) {
-  if (FLAG == -1 || FLAG == 0) return fdiv(1 + 0.5 * z - 0.25 * z * z, 1 + z + 0.25 * z * z);
-  if (FLAG == 1) return fdiv(1 + z, 1 + z + 0.25 * z * z);
-  if (FLAG == 2) return 1.0;     // (1 + z/2) / (1 + z/2)
-  return fdiv(1.0, 1 + 0.5 * z);
-}
-#else
+#if !MBM_FAST_ARITH
 // Damping factors of the direct production integration (src/Flux.c:213-223) at one
 // argument: flags 0 (= -1) and 1 share a denominator, hence one reciprocal; flag 2 is
 // (1 + z/2) / (1 + z/2), which is 1 in any rounding; flag 3 is a reciprocal.  For
@@ -328,6 +266,7 @@ __device__ __forceinline__ double coll_of(const double (&P)[NV], double dt, cons
   return quotient(nu0 * P[0] * fsqrt(P[3]), Kn) * dt;
 }
 
+#if !MBM_FAST_ARITH
 // ProductionsDirect (src/Flux.c:230-267) with ExternalForce (src/Scenario.c:28-42;
 // force (F, 0)), starting from the primitives P of the input moments, given its damping
 // factors d1 = rdamp<FLAG>(z), d2 = rdamp<FLAG>(2z/3).  Writes the relaxed moments.
@@ -355,36 +294,25 @@ __device__ __forceinline__ void relax_d(const double (&P)[NV], double (&Out)[NV]
 __device__ __forceinline__ void relax_m1(const double (&P)[NV], double (&Out)[NV], double dt,
                                          const Recip& Kn, double F) {
   const double coll = coll_of(P, dt, Kn);
-#if MBM_FAST_ARITH
-  const double d1 = rdamp<-1>(coll), d2 = rdamp<-1>(2.0 / 3 * coll);
-#else
   double d1, d2, unused;
   damp01(coll, d1, unused);
   damp01(2.0 / 3 * coll, d2, unused);
-#endif
   relax_d<-1>(P, Out, dt, F, d1, d2);
 }
+#endif
 
 #if MBM_FAST_ARITH
-// Primitive(relax<FLAG>(P)) in primitive form (fast arithmetic): rho and theta kept,
-// the velocity pushed by dt F for flags 0 and 2, T_ij - theta delta_ij scaled by
-// R(z), q by R(2z/3) -- without forming the moments and dividing by rho again
-template <int FLAG>
-__device__ __forceinline__ void relax_prim(const double (&P)[NV], double (&Q)[NV], double dt,
-                                           const Recip& Kn, double F) {
-  const double rho = P[0], th = P[3];
-  const double coll = rho * fsqrt(th) * Kn.r * dt;
-  const double d1 = rdamp<FLAG>(coll);
-  const double d2 = rdamp<FLAG>(2.0 / 3 * coll);
-  Q[0] = rho;
-  Q[1] = P[1] + ((FLAG == 0 || FLAG == 2) ? dt * F : 0.0);
-  Q[2] = P[2];
-  Q[3] = th;
-  Q[4] = d1 * (P[4] - th) + th;
-  Q[5] = d1 * P[5];
-  Q[6] = d1 * (P[6] - th) + th;
-  Q[7] = d2 * P[7];
-  Q[8] = d2 * P[8];
+// The projection of stage 2 (flag 3) in primitive form: rho, theta and the velocity kept,
+// T_ij - theta delta_ij scaled by 1/(1 + z/2), q by 1/(1 + z/3) -- without forming the
+// moments and dividing by rho again
+__device__ __forceinline__ void project3(double (&P)[NV], double z) {
+  const double th = P[3];
+  const double d1 = frcp(fma(0.5, z, 1.0)), d2 = frcp(fma(0.5, 2.0 / 3 * z, 1.0));
+  P[4] = fma(d1, P[4] - th, th);
+  P[5] = d1 * P[5];
+  P[6] = fma(d1, P[6] - th, th);
+  P[7] = d2 * P[7];
+  P[8] = d2 * P[8];
 }
 #endif
 
@@ -413,8 +341,22 @@ __device__ __forceinline__ void relaxed_moments(const double (&P)[NV], double d1
                                                 double (&Out)[NV]) {
   const double rho = P[0], v1 = P[1], v2 = P[2], th = P[3];
   const double E = rho * fma(0.5, fma(v1, v1, v2 * v2), 1.5 * th);
-  moments_e(rho, v1, v2, E, fma(d1, P[4] - th, th), d1 * P[5], fma(d1, P[6] - th, th), d2 * P[7], d2 * P[8],
-            Out);
+  const double T11 = fma(d1, P[4] - th, th), T12 = d1 * P[5], T22 = fma(d1, P[6] - th, th);
+  Out[0] = rho;
+  Out[1] = rho * v1;
+  Out[2] = rho * v2;
+  Out[3] = E;
+  Out[4] = rho * (T11 + v1 * v1);
+  Out[5] = rho * (T12 + v1 * v2);
+  Out[6] = rho * (T22 + v2 * v2);
+  Out[7] = fma(rho, fma(T11, v1, T12 * v2), fma(E, v1, d2 * P[7]));
+  Out[8] = fma(rho, fma(T12, v1, T22 * v2), fma(E, v2, d2 * P[8]));
+}
+
+__device__ __forceinline__ void relax_m1(const double (&P)[NV], double (&Out)[NV], double dt,
+                                         const Recip& Kn, double) {
+  const Damp01 dm(coll_of(P, dt, Kn));
+  relaxed_moments(P, dm.d1_0, dm.d2_0, Out);
 }
 
 // relax<2>(Primitive(U)) in moment form (fast arithmetic): flag 2 leaves T and q as
@@ -431,13 +373,24 @@ __device__ __forceinline__ void push_moments(const double (&U)[NV], double g, do
   R[4] = fma(g, fma(2.0, U[1], rg), U[4]);
   R[5] = fma(g, U[2], U[5]);
   R[6] = U[6];
-  R[7] = fma(g, U[3] + U[4] + 0.5 * g * fma(3.0, U[1], rg), U[7]);
+  R[7] = fma(g, fma(0.5 * g, fma(3.0, U[1], rg), U[3] + U[4]), U[7]);
   R[8] = fma(g, fma(0.5 * g, U[2], U[5]), U[8]);
 }
 // The same push applies to any moment vector whose temperature and heat flux stay
 // fixed: relax<0>(P) = push_moments(relax<-1>(P), dt F), flag 0 differing from flag
 // -1 only by the force acting on the velocity before the moments are formed.
 #endif
+
+// A cell's update from its relaxation terms and its faces' fluxes, in the order of the
+// reference's face loop (src/Main.c:353-384)
+__device__ __forceinline__ double accumulate(double R, double dtdx, double dtdy, double Fm, double Gm, double G,
+                                             double F) {
+#if MBM_FAST_ARITH
+  return fma(-dtdx, F, fma(-dtdy, G, fma(dtdy, Gm, fma(dtdx, Fm, R))));
+#else
+  return (((R + dtdx * Fm) + dtdy * Gm) - dtdy * G) - dtdx * F;
+#endif
+}
 
 // Limit1 (src/Limiter.c:26-59)
 __device__ __forceinline__ double superbee_phi(double r) {
@@ -456,27 +409,31 @@ __device__ __forceinline__ double limit(double d1, double d2) {
   if (LIM == 3) return d1 * superbee_phi(fdiv(d2, d1));
   const double eps = 1.0e-10;
   const double w1 = fabs(d1) + eps, w2 = fabs(d2) + eps;
+#if MBM_FAST_ARITH
+  return fdiv(fma(w1, d2, w2 * d1), w1 + w2);
+#else
   return fdiv(w1 * d2 + w2 * d1, w1 + w2);
+#endif
 }
 
 #if !MBM_FAST_ARITH
-// L = Limit1(d1, d2) and the slope L / h of the nine primitives (src/Main.c:346-349), D =
+// L = Limit1(d1, d2) and the slope L / h of N components (src/Main.c:346-349), D =
 // Recip(h), h in the safe range.  The harmonic limiter's quotient has a denominator of its
-// own, |d1| + |d2| + 2e-10: nine reciprocals without a branch, and one check of the set
+// own, |d1| + |d2| + 2e-10: reciprocals without a branch, and one check of the set
 // (numerators within 2^+-400 or zero, denominators below 2^80, so that L itself is within
 // the range the division by h admits).
-template <int LIM>
-__device__ __forceinline__ void slopes(const double (&d1)[NV], const double (&d2)[NV], const Recip& D,
-                                       double (&S)[NV]) {
+template <int LIM, int N>
+__device__ __forceinline__ void slopes(const double (&d1)[N], const double (&d2)[N], const Recip& D,
+                                       double (&S)[N]) {
   if (LIM == 0) {
 #pragma unroll
-    for (int n = 0; n < NV; n++) S[n] = 0.0;      // 0 / h
+    for (int n = 0; n < N; n++) S[n] = 0.0;      // 0 / h
     return;
   }
-  double L[NV];
+  double L[N];
   if (LIM != 4) {
 #pragma unroll
-    for (int n = 0; n < NV; n++) L[n] = limit<LIM>(d1[n], d2[n]);
+    for (int n = 0; n < N; n++) L[n] = limit<LIM>(d1[n], d2[n]);
     quotients(L, D, S);
     return;
   }
@@ -485,7 +442,7 @@ __device__ __forceinline__ void slopes(const double (&d1)[NV], const double (&d2
   unsigned md = 0u;
   int ones = 0;
 #pragma unroll
-  for (int n = 0; n < NV; n++) {
+  for (int n = 0; n < N; n++) {
     const double w1 = fabs(d1[n]) + eps, w2 = fabs(d2[n]) + eps;
     const double x = w1 * d2[n] + w2 * d1[n], y = w1 + w2;
     g.add(x);
@@ -496,7 +453,7 @@ __device__ __forceinline__ void slopes(const double (&d1)[NV], const double (&d2
   }
   if (__builtin_expect(g.lo < (623u << 21) || g.hi >= (1424u << 21) || md >= (1103u << 20) || ones || D.bad, 0)) {
 #pragma unroll
-    for (int n = 0; n < NV; n++) S[n] = div_ieee(limit<LIM>(d1[n], d2[n]), D.y);
+    for (int n = 0; n < N; n++) S[n] = div_ieee(limit<LIM>(d1[n], d2[n]), D.y);
   }
 }
 #endif
@@ -513,28 +470,28 @@ __device__ __forceinline__ void slopes(const double (&d1)[NV], const double (&d2
 __device__ __forceinline__ void cons_flux_x(const double (&P)[NV], double (&U)[NV], double (&F)[NV]) {
   const double r = P[0], u = P[1], v = P[2], th = P[3];
   const double T11 = P[4], T12 = P[5], T22 = P[6], q1 = P[7], q2 = P[8];
-  const double vs = u * u + v * v;
-  const double E = 0.5 * r * vs + 1.5 * r * th;
+  const double uu = u * u, vs = fma(v, v, uu);
+  const double E = fma(1.5 * r, th, 0.5 * r * vs);
   U[0] = r;
   U[1] = r * u;
   U[2] = r * v;
   U[3] = E;
-  U[4] = r * (T11 + u * u);
+  U[4] = r * (T11 + uu);
   U[5] = r * (T12 + u * v);
-  U[6] = r * (T22 + v * v);
-  U[7] = q1 + E * u + r * (T11 * u + T12 * v);
-  U[8] = q2 + E * v + r * (T12 * u + T22 * v);
+  U[6] = r * fma(v, v, T22);
+  U[7] = fma(r, fma(T11, u, T12 * v), fma(E, u, q1));
+  U[8] = fma(r, fma(T12, u, T22 * v), fma(E, v, q2));
   const double q1a = 1.2 * q1, q1b = 0.4 * q1, q2b = 0.4 * q2;
   const double rT12 = r * T12, t2 = rT12 + rT12;
   F[0] = U[1];
   F[1] = U[4];
   F[2] = U[5];
   F[3] = U[7];
-  F[4] = fma(U[1], fma(3.0, T11, u * u), q1a);
+  F[4] = fma(U[1], fma(3.0, T11, uu), q1a);
   F[5] = fma(v, U[4], fma(u, t2, q2b));
   F[6] = fma(u, U[6], fma(v, t2, q1b));
   F[7] = fma(u, fma(-E, u, 2.0 * U[7]) + q1a,
-             fma(q2b, v, 0.5 * r * fma(T11, vs + 7.0 * th, -2.0 * th * th)));
+             fma(q2b, v, 0.5 * r * fma(T11, fma(7.0, th, vs), -2.0 * th * th)));
   F[8] = fma(1.4, fma(q2, u, q1 * v), fma(u * v, fma(r, T11 + T22, E), rT12 * fma(1.5, vs, 3.5 * th)));
 }
 
@@ -612,6 +569,81 @@ __device__ __forceinline__ double hll(const double (&PL)[NV], const double (&PR)
   for (int n = 0; n < NV; n++) A[n] = kL * f[n];
   conservative(PR, UR);
   flux_normal<DIR>(UR, f);
+  if (pos) {
+    const Recip D(alph);
+    double num[NV];
+#pragma unroll
+    for (int n = 0; n < NV; n++) num[n] = A[n] - lamL * f[n] + lamL * lamR * (UR[n] - UL[n]);
+    quotients(num, D, flx);
+  } else {
+#pragma unroll
+    for (int n = 0; n < NV; n++) flx[n] = 0.5 * (A[n] + f[n]);
+  }
+  return cMax;
+}
+// v, or -v where sg is the sign bit
+__device__ __forceinline__ double signed_by(double v, unsigned sg) {
+  return __hiloint2double(__double2hiint(v) ^ (int)sg, __double2loint(v));
+}
+
+// flux_normal with the direction a run-time value: U and F of a y face come with x and y
+// swapped, so that both directions run the same operations.  An x face rotates by normal
+// (1, 0), tangent (0, -1), a y face by (0, 1), (1, -0): in the swapped order the two differ by
+// the sign of the second component (sg: the sign bit for x faces) and by the sign of the zero
+// products (z: +0 for x, -0 for y faces), each FMA below being the one that flux_normal
+// forms in its direction.
+__device__ __forceinline__ void flux_swapped(const double (&U)[NV], bool y, unsigned sg, double z,
+                                             double (&F)[NV]) {
+  double W[NV], G[NV];
+  W[0] = U[0];
+  W[1] = fma(U[2], 0.0, U[1]);
+  W[2] = fma(U[1], z, signed_by(U[2], sg));
+  W[3] = U[3];
+  const double a = fma(U[5], 0.0, U[4]), b = fma(U[6], 0.0, U[5]);
+  W[4] = fma(b, 0.0, a);
+  W[5] = fma(a, z, signed_by(b, sg));
+  const double a2 = fma(U[4], z, signed_by(U[5], sg)), b2 = fma(U[5], z, signed_by(U[6], sg));
+  W[6] = fma(a2, z, signed_by(b2, sg));
+  W[7] = fma(U[8], 0.0, U[7]);
+  W[8] = fma(U[7], z, signed_by(U[8], sg));
+  grad13_flux_x(W, G);
+  F[0] = G[0];
+  F[1] = fma(G[2], z, G[1]);
+  F[2] = fma(G[1], 0.0, signed_by(G[2], sg));
+  F[3] = G[3];
+  const double a3 = fma(G[5], z, G[4]), b3 = fma(G[6], z, G[5]);
+  F[4] = fma(b3, z, a3);
+  const double g4 = y ? G[6] : G[4], g6 = y ? G[4] : G[6];
+  const double p = fma(g6, 0.0, G[5]), r = fma(G[5], 0.0, g4);
+  F[5] = fma(r, z, signed_by(p, sg));
+  const double a4 = fma(G[4], 0.0, signed_by(G[5], sg)), b4 = fma(G[5], 0.0, signed_by(G[6], sg));
+  F[6] = fma(a4, 0.0, signed_by(b4, sg));
+  F[7] = fma(G[8], z, G[7]);
+  F[8] = fma(G[7], 0.0, signed_by(G[8], sg));
+}
+
+// hll with the direction a run-time value: states and flux of a y face with x and y swapped
+// (Conservative commutes with the swap bit for bit)
+__device__ __forceinline__ double hll_swapped(const double (&PL)[NV], const double (&PR)[NV], bool y,
+                                              double (&flx)[NV]) {
+  const unsigned sg = y ? 0u : 0x80000000u;
+  const double z = __hiloint2double(y ? (int)0x80000000u : 0, 0);
+  const double cR = 2.0 * sqrt(5.0 / 3 * PR[3]);
+  const double cL = 2.0 * sqrt(5.0 / 3 * PL[3]);
+  const double vR = PR[1], vL = PL[1];
+  const double cMax = fabs(0.5 * (vL + vR)) + rmax(cR, cL);
+  const double lamL = rmin(vL - cL, 0.0);
+  const double lamR = rmax(vR + cR, 0.0);
+  const double alph = lamR - lamL;
+  const bool pos = alph > 0.0;
+  double UL[NV], UR[NV], f[NV], A[NV];
+  conservative(PL, UL);
+  flux_swapped(UL, y, sg, z, f);
+  const double kL = pos ? lamR : 1.0;
+#pragma unroll
+  for (int n = 0; n < NV; n++) A[n] = kL * f[n];
+  conservative(PR, UR);
+  flux_swapped(UR, y, sg, z, f);
   if (pos) {
     const Recip D(alph);
     double num[NV];

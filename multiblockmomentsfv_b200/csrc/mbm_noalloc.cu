@@ -36,6 +36,8 @@
 namespace mbm {
 namespace bitwise {
 cudaError_t launch_stage(int lim, const StageArgs& a, int grid, cudaStream_t s);
+cudaError_t launch_tiles(const StageArgs& a, cudaStream_t s);
+int tile_ctas_per_sm();
 int stage_ctas_per_sm(int heun);
 int stage_cta_warps();
 }
@@ -55,7 +57,8 @@ constexpr size_t OFF_BLK = OFF_LAM + sizeof(unsigned long long) * 6 * NOALLOC_MA
 constexpr size_t OFF_WORK = (OFF_BLK + sizeof(BlockDev) * NOALLOC_MAX_BLOCKS + 255) & ~size_t(255);
 constexpr size_t NOALLOC_SCRATCH_BYTES = 320 * 1024;
 constexpr int NOALLOC_MAX_WORK = (int)((NOALLOC_SCRATCH_BYTES - OFF_WORK) / sizeof(Work));
-constexpr int NOALLOC_SEGMENT_ROWS = 32;
+constexpr int NOALLOC_SEGMENT_ROWS = 32;     // the longest segments: what a call must fit with
+constexpr int NOALLOC_MIN_ROWS = 4;
 
 static_assert(sizeof(CaseDev) <= OFF_QUEUE - OFF_CASE, "controller slot too small");
 // the capacity the header and the error message state; a layout change must update them
@@ -97,9 +100,8 @@ extern "C" int mbm_stage_noalloc(const mbm_block_desc* blocks, int nblocks, cons
     return fail(MBM_EINVAL, "mbm_stage_noalloc: bad limiter, Kn or dt (dt must be positive and finite)");
   cudaStream_t s = (cudaStream_t)stream;
 
-  // block table in the layout of include/mbm_b200.h, and the warp work items
-  long long off = 0;
-  int nwork = 0;
+  // block table in the layout of include/mbm_b200.h
+  long long off = 0, longest = 0, strip_rows = 0, tiles = 0;
   for (int b = 0; b < nblocks; b++) {
     const mbm_block_desc& d = blocks[b];
     if (d.nx < 1 || d.ny < 1 || d.nx > (1 << 20) || d.ny > (1 << 20) ||
@@ -116,18 +118,15 @@ extern "C" int mbm_stage_noalloc(const mbm_block_desc* blocks, int nblocks, cons
     h.dy = d.dy;
     off += h.plane * NV;
     const int nfx = h.nxp - 3, nfy = h.nyp - 3;
-    const int strips = (nfx + STRIP - 1) / STRIP;
-    const int segs = (nfy + NOALLOC_SEGMENT_ROWS - 1) / NOALLOC_SEGMENT_ROWS;
-    if (nwork + (long long)strips * segs > NOALLOC_MAX_WORK)
+    const long long strips = (nfx + STRIP - 1) / STRIP;
+    strip_rows += strips * nfy;
+    tiles += strips * ((nfy + TILE_ROWS - 1) / TILE_ROWS);
+    longest += strips * ((nfy + NOALLOC_SEGMENT_ROWS - 1) / NOALLOC_SEGMENT_ROWS);
+    if (longest > NOALLOC_MAX_WORK)
       return fail(MBM_EINVAL, "mbm_stage_noalloc: blocks exceed the scratch limit (" +
                                   std::to_string(NOALLOC_MAX_WORK) + " warp work items: " +
                                   std::to_string(STRIP) + "-column strips x " +
                                   std::to_string(NOALLOC_SEGMENT_ROWS) + "-row segments)");
-    for (int sg = 0; sg < segs; sg++) {
-      const int J0 = 1 + (int)((long long)nfy * sg / segs);
-      const int J1 = 1 + (int)((long long)nfy * (sg + 1) / segs);
-      for (int k = 0; k < strips; k++) h_work[nwork++] = Work{b, 1 + STRIP * k, J0, J1};
-    }
   }
   // the kernel reads in (and data0) while other warps write out: out must share no
   // element with either (an in-place stage would read cells already overwritten)
@@ -162,14 +161,42 @@ extern "C" int mbm_stage_noalloc(const mbm_block_desc* blocks, int nblocks, cons
   BlockDev* dblk = (BlockDev*)(scratch + OFF_BLK);
   Work* dwork = (Work*)(scratch + OFF_WORK);
 
-  cudaError_t e = cudaSuccess;
+  // Work items: tiles where the grid has few rows of strips, else the row march with segments
+  // that fill one wave of its resident warps, between 4 and 32 rows (32-row segments left a
+  // 777 x 391 block with 364 items for 1,184 warps).  Segments grow until the table fits.
+  int sm = 0;
+  cudaError_t e = cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
+  const int cw = bitwise::stage_cta_warps();
+  const long long ctas = (long long)sm * bitwise::stage_ctas_per_sm(heun);
+  const bool tiled = bitwise::tile_ctas_per_sm() > 0 && tiles <= TILE_MOST_EXACT && tiles <= NOALLOC_MAX_WORK;
+  long long seg = TILE_ROWS;
+  if (!tiled) {
+    seg = std::max<long long>(NOALLOC_MIN_ROWS, (strip_rows + ctas * cw - 1) / std::max<long long>(1, ctas * cw));
+    seg = std::min<long long>(seg, NOALLOC_SEGMENT_ROWS);
+  }
+  int nwork = 0;
+  for (;; seg++) {
+    long long n = 0;
+    for (int b = 0; b < nblocks; b++)
+      n += (long long)((h_blk[b].nxp - 3 + STRIP - 1) / STRIP) * ((h_blk[b].nyp - 3 + seg - 1) / seg);
+    if (n <= NOALLOC_MAX_WORK) break;      // at 32 rows it does
+  }
+  for (int b = 0; b < nblocks; b++) {
+    const int nfx = h_blk[b].nxp - 3, nfy = h_blk[b].nyp - 3;
+    const int strips = (nfx + STRIP - 1) / STRIP, segs = (int)((nfy + seg - 1) / seg);
+    for (int sg = 0; sg < segs; sg++) {
+      // tiles of TILE_ROWS rows, or segments of equal length
+      const int J0 = 1 + (tiled ? sg * TILE_ROWS : (int)((long long)nfy * sg / segs));
+      const int J1 = tiled ? J0 + TILE_ROWS : 1 + (int)((long long)nfy * (sg + 1) / segs);
+      for (int k = 0; k < strips; k++) h_work[nwork++] = Work{b, 1 + STRIP * k, J0, J1};
+    }
+  }
+
   if (!e) e = cudaMemcpyAsync(dcase, &h_case, sizeof(CaseDev), cudaMemcpyHostToDevice, s);
   if (!e) e = cudaMemcpyAsync(dblk, h_blk, sizeof(BlockDev) * nblocks, cudaMemcpyHostToDevice, s);
   if (!e) e = cudaMemcpyAsync(dwork, h_work, sizeof(Work) * nwork, cudaMemcpyHostToDevice, s);
   if (!e) e = cudaMemsetAsync(dqueue, 0, sizeof(int), s);
   if (!e) e = cudaMemsetAsync(dlam, 0, sizeof(unsigned long long) * 6 * nblocks, s);
-  int sm = 0;
-  if (!e) e = cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
   if (e) return fail(MBM_ECUDA, cudaGetErrorString(e));
 
   StageArgs a{};
@@ -186,9 +213,8 @@ extern "C" int mbm_stage_noalloc(const mbm_block_desc* blocks, int nblocks, cons
   a.sel_in = SEL_CUR;
   a.sel_d0 = heun ? SEL_TMP : SEL_CUR;
   a.sel_out = SEL_OTHER;
-  const int cw = bitwise::stage_cta_warps();
-  const long long grid = std::min<long long>((nwork + cw - 1) / cw, (long long)sm * bitwise::stage_ctas_per_sm(heun));
-  e = bitwise::launch_stage(limiter, a, (int)grid, s);
+  e = tiled ? bitwise::launch_tiles(a, s)
+            : bitwise::launch_stage(limiter, a, (int)std::min<long long>((nwork + cw - 1) / cw, ctas), s);
   if (!e) e = cudaMemcpyAsync(h_lam, dlam, sizeof(unsigned long long) * 6 * nblocks, cudaMemcpyDeviceToHost, s);
   if (!e) e = cudaMemcpyAsync(&h_nonfinite, (const unsigned char*)dcase + offsetof(CaseDev, nonfinite), sizeof(int),
                               cudaMemcpyDeviceToHost, s);

@@ -192,7 +192,7 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
   const bool col_cell = C >= 1 && C <= nxp - 2;      // relaxation range (src/Main.c:320-321)
   const bool col_out = lane >= 2 && lane <= 29 && C >= NG && C <= nxp - 1 - NG;
   const bool ylane = lane >= 2 && lane <= 29;        // owners of this strip's y faces
-  const double dtdx = dt / B.dx, dtdy = dt / B.dy;
+  const double dtdx = div_rn(dt, B.dx), dtdy = div_rn(dt, B.dy);
 #if !MBM_FAST_ARITH
   const Recip rdx(B.dx), rdy(B.dy);   // dx, dy in the safe range (checked at creation)
   const double hdx = 0.5 * B.dx, hdy = 0.5 * B.dy;
@@ -317,7 +317,7 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
         // stage 1: one collision number and one reciprocal per damping argument serve
         // the CFL share (flag 0), the relaxation term of the update (flag -1, stored for
         // the update of this row and for stage 2) and the projection (flag 1)
-        const Damp01 dm(Q[0] * fsqrt(Q[3]) * Kn.r * dt);
+        const Damp01 dm(coll_of(Q, dt, Kn));
         if (ok && col_cell && r >= 1 && r <= nyp - 2) {
           const double c = 0.5 * (1 - dm.d2_0);
           if (c > prod) prod = c;
@@ -376,12 +376,8 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
 #endif
       if (!(col_ring || r == 0 || r == nyp - 1)) {
 #if MBM_FAST_ARITH
-        if (HEUN == 1) {   // stage 2 (flag 3): no CFL share (flag 2 is the identity)
-          double V[NV];
-          relax_prim<3>(Q, V, dt, Kn, Fx);
-#pragma unroll
-          for (int n = 0; n < NV; n++) Q[n] = V[n];
-        }
+        // stage 2 (flag 3): no CFL share (flag 2 is the identity)
+        if (HEUN == 1) project3(Q, coll_of(Q, dt, Kn));
 #else
         double V[NV];
         relax_d<2 * HEUN + 1>(Q, V, dt, Fx, d1p, d2p);
@@ -535,11 +531,7 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
         }
 #pragma unroll
         for (int n = 0; n < NV; n++) {
-          double v = R[n];
-          v += dtdx * Fm[n];
-          v += dtdy * win.G[n][lane];
-          v -= dtdy * G[n];
-          v -= dtdx * F[n];
+          double v = accumulate(R[n], dtdx, dtdy, Fm[n], win.G[n][lane], G[n], F[n]);
           if (HEUN == 1) v = 0.5 * v;
           out[n * plane + idx] = v;
           expmax = max(expmax, __double2hiint(v) & 0x7ff00000);
