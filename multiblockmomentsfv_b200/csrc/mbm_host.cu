@@ -626,7 +626,7 @@ static int autotune(mbm_ctx* c) {
   int limmix = 0;
   for (const LimGroup& g : c->groups[0]) limmix |= 1 << g.lim;
   const auto key = std::make_tuple(strip_rows, c->nblk, limmix,
-                                   (c->ctas_per_sm[0] * 256 + c->ctas_per_sm[1]) * c->cta_warps);
+                                   ((c->ctas_per_sm[0] * 256 + c->ctas_per_sm[1]) * c->cta_warps) * 2 + c->fast);
   {
     std::lock_guard<std::mutex> g(g_tune_mu);
     auto it = g_tune_cache.find(key);

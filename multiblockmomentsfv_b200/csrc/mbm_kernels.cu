@@ -5,10 +5,6 @@
 #include <stdint.h>
 
 #include "mbm_internal.h"
-// the bitwise kernel's unfused arithmetic needs more registers than the fast one: two
-// CTAs per SM (238 / 226 registers, no spills) run a 4 x 1024^2 step in 1.96 ms, three (168,
-// spilling 40-64 bytes) in 2.01 ms, and 4 x 256^2 in 0.196 against 0.232 ms
-#define STAGE_MIN_CTAS 2
 #include "mbm_tile.cuh"    // the stage kernels in namespace mbm::bitwise
 
 namespace mbm {

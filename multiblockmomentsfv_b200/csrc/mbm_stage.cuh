@@ -1,6 +1,6 @@
-// mbm_stage.cuh -- the Heun stage kernel (Update, src/Main.c:297-396), compiled once per
-// arithmetic mode: mbm_kernels.cu instantiates it in namespace mbm::bitwise (with
-// -fmad=false), mbm_stage_fast.cu in mbm::fastmath (MBM_FAST_ARITH, -fmad=true).
+// mbm_stage.cuh -- the Heun stage of large grids (Update, src/Main.c:297-396) in fast
+// arithmetic (MBM_FAST_ARITH, mbm_stage_fast.cu), and what its bitwise counterpart
+// (mbm_stage_exact.cuh) and the tiles (mbm_tile.cuh) share with it.
 //
 // One warp owns a strip of 28 output columns plus a 2-column halo on each side
 // (lane l <-> column I0 - 2 + l) and a segment of rows, and marches up the segment.
@@ -42,6 +42,67 @@ __device__ __forceinline__ void load_cell(const double* __restrict__ base, long 
   for (int n = 0; n < NV; n++) U[n] = __ldg(base + n * plane + idx);
 }
 
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t));
+  return t;
+}
+// per-thread asynchronous 8-byte copy global -> shared (cp.async), and its groups
+__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_one() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+
+// the largest of a warp's values, as bits; the values are >= +0 (a NaN never passed a '>'
+// test), so their bit patterns order like the values: the largest high word, then the largest
+// low word among those that have it
+__device__ __forceinline__ unsigned long long warp_max(double v) {
+  const unsigned h = (unsigned)__double2hiint(v), hm = __reduce_max_sync(0xffffffffu, h);
+  const unsigned lm = __reduce_max_sync(0xffffffffu, h == hm ? (unsigned)__double2loint(v) : 0u);
+  return (unsigned long long)hm << 32 | lm;
+}
+
+// a warp's share of the per-block maxima and of failure detection (a NaN or infinity in a
+// written cell marks the case); the values are >= 0 (a NaN never passed a '>' test), so their
+// bit patterns order like the values
+template <int HEUN>
+__device__ __forceinline__ void stage_maxima(const StageArgs& a, int blk, int case_id, int lane, double lamx,
+                                             double lamy, double prod, int expmax) {
+  const unsigned long long m[3] = {warp_max(lamx), warp_max(lamy), warp_max(prod)};
+  const bool bad = __any_sync(0xffffffffu, expmax == 0x7ff00000);
+  if (lane != 0) return;
+  unsigned long long* slot = a.lam + ((size_t)blk * 2 + HEUN) * 3;
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+    if (m[k] != 0ull) atomicMax(slot + k, m[k]);
+  if (bad) atomicOr(&a.cases[case_id].nonfinite, 1);
+}
+
+// SetBoundary (src/Boundary.c:173-193) fused into the stage: once a work item's cells
+// are stored, its warp writes the ghost cells whose owners the item wrote, one entry per
+// lane -- the owner's value read back from the output layer, or the Dirichlet row --
+// sign-flipped on the wall components as the gather does
+__device__ __forceinline__ void scatter_item(const StageArgs& a, int wi, int lane, double* base,
+                                             const double* out, long long plane) {
+  const int2 r = a.gs_item[wi];
+  if (r.y <= 0) return;
+  __syncwarp();     // every lane's stores of this item are visible to the warp
+  for (int e = r.x + lane; e < r.x + r.y; e += 32) {
+    const GhostScatter g = a.gs[e];
+    const bool fx = g.flags & 1, fy = (g.flags >> 1) & 1;
+#pragma unroll
+    for (int m = 0; m < NV; m++) {
+      const double v = g.drow < 0 ? out[m * plane + g.src] : __ldg(a.dirichlet + (size_t)g.drow * NV + m);
+      const bool flip = (fx && (m == 1 || m == 5 || m == 7)) != (fy && (m == 2 || m == 5 || m == 8));
+      base[g.dst + m * g.plane] = flip ? -v : v;
+    }
+  }
+}
+
+#if MBM_FAST_ARITH
 // Rolling state of one warp, lane fastest (conflict-free 8-byte accesses): the
 // projected primitives of three consecutive rows, the lower state of the next
 // y face and the y flux of the face below the row being finished.  Stage 2 adds two
@@ -91,11 +152,6 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned 
       : "memory");
   return done != 0;
 }
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t));
-  return t;
-}
 // false when the phase did not complete within 0.25 s of device time (a copy that never
 // lands); at most 65,536 tests of at most 20 us each, should the timer not advance
 __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity) {
@@ -119,14 +175,6 @@ __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory"); }
 constexpr unsigned ROW_BOX_BYTES = NV * 32 * sizeof(double);   // one 32 x 1 x 9 box
 
-// per-thread asynchronous 8-byte copy global -> shared (cp.async), and its groups
-__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_one() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 #ifndef STAGE_CTA_WARPS
 #define STAGE_CTA_WARPS CTA_WARPS   // warps per CTA of this instantiation
 #endif
@@ -139,27 +187,6 @@ constexpr int STAGE_WARPS = STAGE_CTA_WARPS;
 // slots by bulk tensor copies; tma: whether it does (warp-uniform; ph holds the phase
 // bits of the warp's two window barriers across items).  The instantiation without it
 // carries only the per-lane copies: the unused branches alone cost 4 % of stage 2.
-// SetBoundary (src/Boundary.c:173-193) fused into the stage: once a work item's cells
-// are stored, its warp writes the ghost cells whose owners the item wrote, one entry per
-// lane -- the owner's value read back from the output layer, or the Dirichlet row --
-// sign-flipped on the wall components as the gather does
-__device__ __forceinline__ void scatter_item(const StageArgs& a, int wi, int lane, double* base,
-                                             const double* out, long long plane) {
-  const int2 r = a.gs_item[wi];
-  if (r.y <= 0) return;
-  __syncwarp();     // every lane's stores of this item are visible to the warp
-  for (int e = r.x + lane; e < r.x + r.y; e += 32) {
-    const GhostScatter g = a.gs[e];
-    const bool fx = g.flags & 1, fy = (g.flags >> 1) & 1;
-#pragma unroll
-    for (int m = 0; m < NV; m++) {
-      const double v = g.drow < 0 ? out[m * plane + g.src] : __ldg(a.dirichlet + (size_t)g.drow * NV + m);
-      const bool flip = (fx && (m == 1 || m == 5 || m == 7)) != (fy && (m == 2 || m == 5 || m == 8));
-      base[g.dst + m * g.plane] = flip ? -v : v;
-    }
-  }
-}
-
 // Returns false when a bounded wait on a copy ran out: the case is flagged (the
 // controller stops it with a timeout status) and the warp stops taking items.
 template <int HEUN, int LIM, bool TMA>
@@ -176,10 +203,9 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
   const double* __restrict__ in = layer_ptr(a.buf, phys_layer(a.sel_in, cur)) + B.off;
   const double* __restrict__ d0 = layer_ptr(a.buf, phys_layer(a.sel_d0, cur)) + B.off;
   double* __restrict__ out = layer_ptr(a.buf, phys_layer(a.sel_out, cur)) + B.off;
-  // the relaxation term of the stage-1 input (flag -1): written by stage 1 at its row r
-  // (fast arithmetic: read back, with plain loads, by the update of that row two
-  // iterations later); stage 2 reads it with rlx_read in place of forming it from
-  // Data0.  Null (bitwise only): not stored.
+  // the relaxation term of the stage-1 input (flag -1): written by stage 1 at its row r,
+  // read back, with plain loads, by the update of that row two iterations later; stage 2
+  // reads it with rlx_read in place of forming it from Data0
   double* __restrict__ rlx = a.rlx ? a.rlx + B.off : nullptr;
   const bool rlx_rd = HEUN == 1 && a.rlx_read;
   const double* __restrict__ d0src = rlx_rd ? rlx : d0;
@@ -193,10 +219,6 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
   const bool col_out = lane >= 2 && lane <= 29 && C >= NG && C <= nxp - 1 - NG;
   const bool ylane = lane >= 2 && lane <= 29;        // owners of this strip's y faces
   const double dtdx = div_rn(dt, B.dx), dtdy = div_rn(dt, B.dy);
-#if !MBM_FAST_ARITH
-  const Recip rdx(B.dx), rdy(B.dy);   // dx, dy in the safe range (checked at creation)
-  const double hdx = 0.5 * B.dx, hdy = 0.5 * B.dy;
-#endif
   double lamx = 0.0, lamy = 0.0, prod = 0.0;
   int expmax = 0;     // largest exponent field (high word & 0x7ff00000) written: all ones = NaN or inf
 
@@ -312,7 +334,6 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
         u_fetch(r + 1);                      // into the slot just read
       }
       primitive(U, Q);
-#if MBM_FAST_ARITH
       if (HEUN == 0) {
         // stage 1: one collision number and one reciprocal per damping argument serve
         // the CFL share (flag 0), the relaxation term of the update (flag -1, stored for
@@ -340,49 +361,9 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
           Q[8] = dm.d2_1 * Q[8];
         }
       }
-#endif
-#if !MBM_FAST_ARITH
-      // one collision number serves every ProductionsDirect of this cell in this stage,
-      // each flag's damping factors formed from it with the reference's expressions:
-      // the CFL share and the update's relaxation term (flag 2 HEUN, parked in the
-      // output layer until the update of this row two iterations later), stage 1's
-      // relaxation of Data0 for stage 2 (flag -1: flag 0 without the force) and the
-      // projection (flag 2 HEUN + 1)
-      const double z = coll_of(Q, dt, Kn);
-      double d1u, d2u, d1p, d2p;      // flags 2 HEUN and 2 HEUN + 1, at z and 2z/3
-      if (HEUN == 0) {
-        damp01(z, d1u, d1p);
-        damp01(2.0 / 3 * z, d2u, d2p);
-      } else {
-        damp23(z, d1u, d1p);
-        damp23(2.0 / 3 * z, d2u, d2p);
-      }
-      if (ok && col_cell && r >= 1 && r <= nyp - 2) {
-        const double c = 0.5 * (1 - d2u);
-        if (c > prod) prod = c;
-      }
-      if (ok && col_out && r >= NG && r <= nyp - 1 - NG && r >= w.J0 && r < w.J1) {
-        const long long idx = (long long)r * pitch + C + 1;
-        double R[NV];
-        relax_d<2 * HEUN>(Q, R, dt, Fx, d1u, d2u);
-#pragma unroll
-        for (int n = 0; n < NV; n++) out[n * plane + idx] = R[n];
-        if (HEUN == 0 && rlx) {
-          relax_d<-1>(Q, R, dt, Fx, d1u, d2u);
-#pragma unroll
-          for (int n = 0; n < NV; n++) rlx[n * plane + idx] = R[n];
-        }
-      }
-#endif
       if (!(col_ring || r == 0 || r == nyp - 1)) {
-#if MBM_FAST_ARITH
         // stage 2 (flag 3): no CFL share (flag 2 is the identity)
         if (HEUN == 1) project3(Q, coll_of(Q, dt, Kn));
-#else
-        double V[NV];
-        relax_d<2 * HEUN + 1>(Q, V, dt, Fx, d1p, d2p);
-        primitive(V, Q);
-#endif
       }
 #pragma unroll
       for (int n = 0; n < NV; n++) win.P[s0][n][lane] = Q[n];
@@ -392,7 +373,6 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
     const bool face_now = r >= rs + 3;
     if (r >= rs + 2) {
       double hi[NV], S[NV];
-#if MBM_FAST_ARITH
       // the face states P -+ (dy/2) (L/dy) are P -+ L/2: dy cancels
 #pragma unroll
       for (int n = 0; n < NV; n++) {
@@ -405,24 +385,6 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
         hi[n] = fma(-0.5, S[n], p0);
         G[n] = fma(0.5, S[n], p0);            // lower state of the next face, parked in G
       }
-#else
-      {
-        double d1[NV], d2[NV];
-#pragma unroll
-        for (int n = 0; n < NV; n++) {
-          const double p0 = win.P[sm1][n][lane];
-          d1[n] = p0 - win.P[sm2][n][lane];
-          d2[n] = win.P[s0][n][lane] - p0;
-        }
-        slopes<LIM>(d1, d2, rdy, S);
-      }
-#pragma unroll
-      for (int n = 0; n < NV; n++) {
-        const double p0 = win.P[sm1][n][lane];
-        hi[n] = p0 - hdy * S[n];
-        G[n] = p0 + hdy * S[n];               // lower state of the next face, parked in G
-      }
-#endif
       if (face_now && ylane) {
         double lo[NV];
 #pragma unroll
@@ -452,7 +414,6 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
       __syncwarp();   // the window row is read across lanes below (other lanes wrote it)
       // the right-hand difference of a lane is its right neighbour's left-hand one (the
       // same subtraction of the same operands), passed down instead of recomputed
-#if MBM_FAST_ARITH
 #pragma unroll
       for (int n = 0; n < NV; n++) {
         P0[n] = win.P[sm2][n][lane];
@@ -464,23 +425,6 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
         lo[n] = fma(0.5, Sx[n], P0[n]);
         hi[n] = __shfl_down_sync(0xffffffffu, fma(-0.5, Sx[n], P0[n]), 1);
       }
-#else
-      {
-        double d1[NV], d2[NV];
-#pragma unroll
-        for (int n = 0; n < NV; n++) {
-          P0[n] = win.P[sm2][n][lane];
-          d1[n] = P0[n] - win.P[sm2][n][(lane + 31) & 31];      // left neighbour (lane 0: unused)
-          d2[n] = __shfl_down_sync(0xffffffffu, d1[n], 1);
-        }
-        slopes<LIM>(d1, d2, rdx, Sx);
-      }
-#pragma unroll
-      for (int n = 0; n < NV; n++) {
-        lo[n] = P0[n] + hdx * Sx[n];
-        hi[n] = __shfl_down_sync(0xffffffffu, P0[n] - hdx * Sx[n], 1);
-      }
-#endif
 #pragma unroll
       for (int n = 0; n < NV; n++) F[n] = 0.0;
       if (lane >= 1 && lane <= 29) {
@@ -494,7 +438,6 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
       if (col_out && J >= NG && J <= nyp - 1 - NG) {
         const long long idx = (long long)J * pitch + C + 1;
         double U[NV], Q[NV], R[NV];
-#if MBM_FAST_ARITH
         const double g = dt * Fx;
         if constexpr (HEUN == 1) {
           load_cell(in, plane, idx, U);
@@ -510,11 +453,6 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
 #pragma unroll
           for (int n = 0; n < NV; n++) R[n] = U[n];
         }
-#else
-        // relax<2 HEUN> of this cell, parked here by the window pass (plain loads)
-#pragma unroll
-        for (int n = 0; n < NV; n++) R[n] = out[n * plane + idx];
-#endif
         if constexpr (HEUN == 1) {
           double R0[NV];
 #pragma unroll
@@ -568,22 +506,7 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
   }
   if (a.gs_item) scatter_item(a, wi, lane, out - B.off, out, plane);
 
-  // per-block maxima; the values are >= 0 (or NaN, which never passes a '>' test
-  // above), so their bit patterns order like the values
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    lamx = fmax(lamx, __shfl_xor_sync(0xffffffffu, lamx, o));
-    lamy = fmax(lamy, __shfl_xor_sync(0xffffffffu, lamy, o));
-    prod = fmax(prod, __shfl_xor_sync(0xffffffffu, prod, o));
-  }
-  // failure detection: a NaN or infinity in a written cell marks the case
-  if (__any_sync(0xffffffffu, expmax == 0x7ff00000) && lane == 0) atomicOr(&a.cases[B.case_id].nonfinite, 1);
-  if (lane == 0) {
-    unsigned long long* slot = a.lam + ((size_t)w.blk * 2 + HEUN) * 3;
-    if (lamx > 0.0) atomicMax(slot + 0, (unsigned long long)__double_as_longlong(lamx));
-    if (lamy > 0.0) atomicMax(slot + 1, (unsigned long long)__double_as_longlong(lamy));
-    if (prod > 0.0) atomicMax(slot + 2, (unsigned long long)__double_as_longlong(prod));
-  }
+  stage_maxima<HEUN>(a, w.blk, B.case_id, lane, lamx, lamy, prod, expmax);
   return true;
 }
 
@@ -611,7 +534,6 @@ __global__ void STAGE_BOUNDS stage_kernel(const StageArgs a) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   bool tma = false, drop = false;
   unsigned ph = 0;
-#if MBM_FAST_ARITH
   if constexpr (HEUN == 1 && TMA) {
     // bulk tensor copies need 128-byte aligned slots (the window layout keeps them so
     // from an aligned base; otherwise the per-lane copies serve)
@@ -630,7 +552,6 @@ __global__ void STAGE_BOUNDS stage_kernel(const StageArgs a) {
       __syncwarp();
     }
   }
-#endif
   for (;;) {
     int w = 0;
     if (lane == 0) w = atomicAdd(a.queue, 1);
@@ -644,7 +565,7 @@ template <int HEUN, int LIM>
 static void smem_attr() {
   cudaFuncSetAttribute(stage_kernel<HEUN, LIM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        stage_smem<HEUN>());
-  if constexpr (HEUN == 1 && MBM_FAST_ARITH != 0)
+  if constexpr (HEUN == 1)
     cudaFuncSetAttribute(stage_kernel<HEUN, LIM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          stage_smem<HEUN>());
 }
@@ -689,11 +610,10 @@ static cudaError_t launch_stage_lim(int lim, const StageArgs& a, int grid, cudaS
 
 cudaError_t launch_stage(int lim, const StageArgs& a, int grid, cudaStream_t s) {
   if (!a.heun) return launch_stage_lim<0, false>(lim, a, grid, s);
-#if MBM_FAST_ARITH
   if (a.tmap) return launch_stage_lim<1, true>(lim, a, grid, s);
-#endif
   return launch_stage_lim<1, false>(lim, a, grid, s);
 }
+#endif
 
 }  // namespace MBM_ARITH
 }  // namespace mbm

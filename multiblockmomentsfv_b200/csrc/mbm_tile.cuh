@@ -33,6 +33,9 @@
 #pragma once
 
 #include "mbm_stage.cuh"
+#if !MBM_FAST_ARITH
+#include "mbm_stage_exact.cuh"
+#endif
 #include "mbm_step.cuh"
 
 namespace mbm {
@@ -61,15 +64,6 @@ struct TileCase {
   int lim, cur;
   bool gather;       // ghost cells of the stage's input are read through the ghost map
 };
-
-// the largest of a warp's values, as bits; the values are >= +0 (a NaN never passed a '>'
-// test), so their bit patterns order like the values: the largest high word, then the largest
-// low word among those that have it
-__device__ __forceinline__ unsigned long long warp_max(double v) {
-  const unsigned h = (unsigned)__double2hiint(v), hm = __reduce_max_sync(0xffffffffu, h);
-  const unsigned lm = __reduce_max_sync(0xffffffffu, h == hm ? (unsigned)__double2loint(v) : 0u);
-  return (unsigned long long)hm << 32 | lm;
-}
 
 // a cell's moments: from the layer, or, for a ghost cell of a gathered layer, from where the
 // ghost fill takes it
