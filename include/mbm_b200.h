@@ -92,7 +92,7 @@ int mbm_destroy(mbm_ctx *ctx);
 
 /* Many independent cases in one context (no counterpart in the reference, which
  * runs one case per process): every Heun stage of every case is one persistent
- * launch per limiter in use, and mbm_steps_batch advances all cases together in
+ * launch, and mbm_steps_batch advances all cases together in
  * one CUDA-graph loop, each with its own dt, t and step count.  Blocks are indexed
  * globally in the transfer calls. */
 int mbm_create_batch(const mbm_block_desc *blocks, int nblocks, const mbm_case_desc *cases,
@@ -286,8 +286,8 @@ int mbm_ghost_scatter(mbm_ctx *ctx, int *on);
 /* *on = 1 when the step loop's kernels (stages, ghost fills, controller) are launched
  * with programmatic dependent launch: each may be scheduled while the one before it
  * finishes and waits on the device for its results, which takes the launch gaps out
- * of the step.  Off with MBM_PDL=0 at context creation, when a stage runs as several
- * limiter groups on forked streams, and when the step graph cannot be built with it.
+ * of the step.  Off with MBM_PDL=0 at context creation and when the step graph cannot be
+ * built with it.
  * A small grid's step loop is one kernel (MBM_TILES=0 at creation: never); *on then
  * tells of its other launches.  No counterpart in the reference. */
 int mbm_dependent_launch(mbm_ctx *ctx, int *on);

@@ -80,11 +80,6 @@ namespace mbm {
 void set_global_error(const std::string& msg) { g_create_error = msg; }
 }  // namespace mbm
 
-struct LimGroup {      // the work items of every block whose case uses one limiter
-  int lim, start, count;
-  int grid[2];         // persistent grid of each Heun stage
-};
-
 struct mbm_ctx {
   mbm_params prm{};
   int device = 0;
@@ -127,7 +122,8 @@ struct mbm_ctx {
   Work* dwork = nullptr;            // the work tables of the two Heun stages, max_items apart
   long long max_items = 0;
   int nwork[2] = {0, 0};
-  std::vector<LimGroup> groups[2];  // limiter groups of each stage's table
+  int grid[2] = {0, 0};             // CTAs of each stage's launch
+  int lim = 0;                      // the limiter of every case, or LIM_ANY
   int nsm = 0, cta_warps = CTA_WARPS;   // stage kernel: warps per CTA
   int ctas_per_sm[2] = {1, 1};          // stage kernel: resident CTAs per SM of each Heun stage
   double seg_rows[2] = {0, 0};      // rows per work item of each Heun stage (ceil(rows / seg_rows) segments)
@@ -139,20 +135,16 @@ struct mbm_ctx {
   double* dcfl = nullptr;           // per-block stage CFL for mbm_update
   double* hcfl = nullptr;           // pinned
   cudaEvent_t ev = nullptr;
-  // limiter groups of one stage run concurrently: forked from `stream`, joined back
-  cudaStream_t aux[4] = {};
   // output staged on the device and copied to the host beside the next interval
   double* out_stage = nullptr;
   std::vector<size_t> out_off;     // bytes, per block (room for the Float64 payload)
   cudaStream_t out_stream = nullptr;
   cudaEvent_t out_ev = nullptr;
-  cudaEvent_t fork_ev = nullptr, join_ev[4] = {};
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
   bool host_loop = false;           // MBM_HOST_LOOP=1: drive the step loop from the host
   // the step loop's kernels launched with programmatic dependent launch (MBM_PDL=0: off;
-  // off too when a stage runs as several limiter groups on forked streams, or when the
-  // step graph cannot be built with it)
+  // off too when the step graph cannot be built with it)
   bool pdl = true;
   bool adjoint = false;             // graph body records checkpoints and dt (mbm_params.adjoint)
   bool fast = false;                // MBM_MODE_FAST: the fastmath stage kernel
@@ -369,34 +361,20 @@ static int resolve_ghosts(const mbm_block_desc* B, int nb, std::vector<Resolved>
 // ------------------------------------------------------------------ create --
 static int pitch_of(int nxp) { return (nxp + 1 + 3) & ~3; }
 
-// Work items grouped by limiter (the stage kernel is specialised per limiter):
-// blocks of cases with limiter L fill group L, strips within row segments.  Each Heun
-// stage has its own table (the autotuner picks each stage's segment length).
-static void build_work(mbm_ctx* c, double seg_rows, std::vector<Work>& w, std::vector<LimGroup>& groups) {
+// Work items: the strips within the row segments of every block.  Each Heun stage has its own
+// table (the autotuner picks each stage's segment length).
+static void build_work(mbm_ctx* c, double seg_rows, std::vector<Work>& w) {
   w.clear();
-  groups.clear();
-  for (int lim = 0; lim < 5; lim++) {
-    const int start = (int)w.size();
-    for (int b = 0; b < c->nblk; b++) {
-      if (c->hcase[c->blk_case[b]].limiter != lim) continue;
-      const int nxp = c->hblk[b].nxp, nyp = c->hblk[b].nyp;
-      const int nfx = nxp - 3, nfy = nyp - 3;          // face positions 1 .. nxp-3 / nyp-3
-      const int strips = (nfx + STRIP - 1) / STRIP;
-      const int segs = std::max(1, (int)std::ceil(nfy / seg_rows - 1e-9));
-      for (int s = 0; s < segs; s++) {
-        // equal-sized segments over face rows [1, nyp-3], the last one reaching nyp-2
-        const int J0 = 1 + (int)((long long)nfy * s / segs);
-        const int J1 = 1 + (int)((long long)nfy * (s + 1) / segs);
-        for (int k = 0; k < strips; k++) w.push_back(Work{b, 1 + STRIP * k, J0, J1});
-      }
-    }
-    const int count = (int)w.size() - start;
-    if (count > 0) {
-      LimGroup g{lim, start, count, {0, 0}};
-      for (int h = 0; h < 2; h++)
-        g.grid[h] = (int)std::min<long long>((count + c->cta_warps - 1) / c->cta_warps,
-                                             (long long)c->nsm * c->ctas_per_sm[h]);
-      groups.push_back(g);
+  for (int b = 0; b < c->nblk; b++) {
+    const int nxp = c->hblk[b].nxp, nyp = c->hblk[b].nyp;
+    const int nfx = nxp - 3, nfy = nyp - 3;          // face positions 1 .. nxp-3 / nyp-3
+    const int strips = (nfx + STRIP - 1) / STRIP;
+    const int segs = std::max(1, (int)std::ceil(nfy / seg_rows - 1e-9));
+    for (int s = 0; s < segs; s++) {
+      // equal-sized segments over face rows [1, nyp-3], the last one reaching nyp-2
+      const int J0 = 1 + (int)((long long)nfy * s / segs);
+      const int J1 = 1 + (int)((long long)nfy * (s + 1) / segs);
+      for (int k = 0; k < strips; k++) w.push_back(Work{b, 1 + STRIP * k, J0, J1});
     }
   }
 }
@@ -458,8 +436,10 @@ static int set_segments(mbm_ctx* c, double seg, int h = -1) {
   for (int k = 0; k < 2; k++) {
     if (h >= 0 && k != h) continue;
     std::vector<Work> work;
-    build_work(c, seg, work, c->groups[k]);
+    build_work(c, seg, work);
     c->nwork[k] = (int)work.size();
+    c->grid[k] = (int)std::min<long long>((c->nwork[k] + c->cta_warps - 1) / c->cta_warps,
+                                          (long long)c->nsm * c->ctas_per_sm[k]);
     CK(cudaMemcpyAsync(c->dwork + k * c->max_items, work.data(), sizeof(Work) * work.size(), cudaMemcpyHostToDevice,
                        c->stream));
     const int st = set_item_scatter(c, k, work);
@@ -494,19 +474,19 @@ static int set_tiles(mbm_ctx* c) {
   for (int h = 0; h < 2; h++) {
     c->nwork[h] = (int)w.size();
     c->seg_rows[h] = TILE_ROWS;
-    c->groups[h].assign(1, LimGroup{0, 0, (int)w.size(), {c->tile_grid, c->tile_grid}});
+    c->grid[h] = c->tile_grid;
   }
   CK(cudaMemcpyAsync(c->dwork, w.data(), sizeof(Work) * w.size(), cudaMemcpyHostToDevice, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   return MBM_OK;
 }
 
-// one Heun stage of every block: one persistent launch per limiter group
-// (with several limiter groups, group k > 0 runs on aux stream k-1, so that one
-// group's CTAs fill the SMs another group's tail leaves idle).  rlx_read (stage 2):
-// the relaxation term of Data0 is read from what the stage 1 of the same attempt
-// stored, instead of being formed again -- only where that stage 1 ran on the same
-// Data0 just before.
+// One Heun stage of every block, one launch: a kernel specialised for the limiter where every
+// case has the same, else one that takes each block's at run time.  (A launch per limiter, on
+// forked streams: 12 cases of five limiters, n up to 320, 370 us a step attempt fast and 947
+// bitwise; one launch 357 and 880.)  rlx_read (stage 2): the relaxation term of Data0 is read from what the
+// stage 1 of the same attempt stored, instead of being formed again -- only where that stage 1
+// ran on the same Data0 just before.
 static cudaError_t launch_stages(mbm_ctx* c, int heun, int sel_in, int sel_d0, int sel_out, int rlx_read,
                                  double* const* bufs = nullptr, bool fill = false) {
   if (c->tiles) {
@@ -517,41 +497,23 @@ static cudaError_t launch_stages(mbm_ctx* c, int heun, int sel_in, int sel_d0, i
     a.rlx_read = heun == 1 && rlx_read;
     return c->fast ? fastmath::launch_tiles(a, c->stream) : bitwise::launch_tiles(a, c->stream);
   }
-  const std::vector<LimGroup>& groups = c->groups[heun];
-  const int ng = (int)groups.size();
-  cudaError_t e0;
-  if (ng > 1) {
-    if ((e0 = cudaEventRecord(c->fork_ev, c->stream))) return e0;
-    for (int k = 1; k < ng; k++)
-      if ((e0 = cudaStreamWaitEvent(c->aux[k - 1], c->fork_ev, 0))) return e0;
+  StageArgs a = stage_args(c, heun, bufs);
+  a.work = c->dwork + heun * c->max_items;
+  a.nwork = c->nwork[heun];
+  a.queue = c->dqueue + heun * 5;
+  a.sel_in = sel_in; a.sel_d0 = sel_d0; a.sel_out = sel_out;
+  a.rlx_read = heun == 1 && rlx_read;
+  // bulk tensor copies: fast stage 2 on the context's own layers (the maps cover TMP
+  // and rlx; the adjoint's recomputation passes other buffers and keeps cp.async)
+  a.tmap = (c->fast && a.rlx_read && !bufs) ? c->dtmap : nullptr;
+  if (a.tmap) a.tma_drop = c->dtma_drop;   // consumed on the device by the first launch
+  if (fill && c->gscatter) {                // the output layer's ghost fill, scattered
+    a.gs_item = c->dgs_item + heun * c->max_items;
+    a.gs = c->dgs + heun * c->gs_ent.size();
+    a.dirichlet = c->ddir;
   }
-  for (int k = 0; k < ng; k++) {
-    const LimGroup& g = groups[k];
-    cudaStream_t st = k == 0 ? c->stream : c->aux[k - 1];
-    StageArgs a = stage_args(c, heun, bufs);
-    a.work = c->dwork + heun * c->max_items + g.start;
-    a.nwork = g.count;
-    a.queue = c->dqueue + heun * 5 + g.lim;
-    a.sel_in = sel_in; a.sel_d0 = sel_d0; a.sel_out = sel_out;
-    a.rlx_read = heun == 1 && rlx_read;
-    // bulk tensor copies: fast stage 2 on the context's own layers (the maps cover TMP
-    // and rlx; the adjoint's recomputation passes other buffers and keeps cp.async)
-    a.tmap = (c->fast && a.rlx_read && !bufs) ? c->dtmap : nullptr;
-    if (a.tmap) a.tma_drop = c->dtma_drop;   // consumed on the device by the first launch
-    if (fill && c->gscatter) {                // the output layer's ghost fill, scattered
-      a.gs_item = c->dgs_item + heun * c->max_items + g.start;
-      a.gs = c->dgs + heun * c->gs_ent.size();
-      a.dirichlet = c->ddir;
-    }
-    cudaError_t e = c->fast ? fastmath::launch_stage(g.lim, a, g.grid[heun], st)
-                            : bitwise::launch_stage(g.lim, a, g.grid[heun], st);
-    if (e != cudaSuccess) return e;
-  }
-  for (int k = 1; k < ng; k++) {
-    if ((e0 = cudaEventRecord(c->join_ev[k - 1], c->aux[k - 1]))) return e0;
-    if ((e0 = cudaStreamWaitEvent(c->stream, c->join_ev[k - 1], 0))) return e0;
-  }
-  return cudaSuccess;
+  return c->fast ? fastmath::launch_stage(c->lim, a, c->grid[heun], c->stream)
+                 : bitwise::launch_stage(c->lim, a, c->grid[heun], c->stream);
 }
 
 // programmatic dependent launch for the launches this thread makes while in scope
@@ -564,7 +526,7 @@ struct PdlScope {
 // fills inside the stage kernels when they scatter them)
 static cudaError_t launch_attempt(mbm_ctx* c, cudaGraphConditionalHandle h, int use_handle) {
   // the attempt's launches use programmatic dependent launch; the thread's others do not
-  PdlScope pdl_scope(c->pdl && c->groups[0].size() <= 1 && c->groups[1].size() <= 1);
+  PdlScope pdl_scope(c->pdl);
   cudaError_t e;
   const bool g = !c->gscatter;
   if ((e = launch_stages(c, 0, SEL_CUR, SEL_CUR, SEL_TMP, 0, nullptr, true))) return e;
@@ -623,9 +585,7 @@ static int autotune(mbm_ctx* c) {
     strip_rows += (long long)((d.nxp - 3 + STRIP - 1) / STRIP) * (d.nyp - 3);
     cells += (long long)d.nxp * d.nyp;
   }
-  int limmix = 0;
-  for (const LimGroup& g : c->groups[0]) limmix |= 1 << g.lim;
-  const auto key = std::make_tuple(strip_rows, c->nblk, limmix,
+  const auto key = std::make_tuple(strip_rows, c->nblk, c->lim,
                                    ((c->ctas_per_sm[0] * 256 + c->ctas_per_sm[1]) * c->cta_warps) * 2 + c->fast);
   {
     std::lock_guard<std::mutex> g(g_tune_mu);
@@ -825,9 +785,7 @@ extern "C" int mbm_create_batch(const mbm_block_desc* blocks, int nblocks, const
 static bool tiles_pay(const mbm_ctx* c, long long tiles) {
   const char* env = getenv("MBM_TILES");
   if (env) return atoi(env) != 0;
-  bool one = true;
-  for (int k = 1; k < c->ncase; k++) one = one && c->hcase[k].limiter == c->hcase[0].limiter;
-  return tiles <= (c->fast ? TILE_MOST_FAST : one ? TILE_MOST_EXACT : TILE_MOST_EXACT_BATCH);
+  return tiles <= (c->fast ? TILE_MOST_FAST : c->lim == LIM_ANY ? TILE_MOST_EXACT_BATCH : TILE_MOST_EXACT);
 }
 
 static int create_impl(const std::vector<mbm_block_desc>& glob, const std::vector<int>& blk_case,
@@ -873,11 +831,6 @@ static int create_impl(const std::vector<mbm_block_desc>& glob, const std::vecto
     c->own_stream = true;
   }
   CKC(cudaEventCreateWithFlags(&c->ev, cudaEventDisableTiming));
-  CKC(cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming));
-  for (int k = 0; k < 4; k++) {
-    CKC(cudaStreamCreateWithFlags(&c->aux[k], cudaStreamNonBlocking));
-    CKC(cudaEventCreateWithFlags(&c->join_ev[k], cudaEventDisableTiming));
-  }
 
   // block table and layer layout
   long long off = 0, max_cells = 0;
@@ -1007,6 +960,7 @@ static int create_impl(const std::vector<mbm_block_desc>& glob, const std::vecto
     h.blk0 = cases[k].first_block;
     h.nblk = cases[k].nblocks;
     h.max_attempts = c->prm.max_attempts;
+    c->lim = k == 0 || h.limiter == c->lim ? h.limiter : LIM_ANY;
   }
   CKC(cudaMemcpyAsync(c->dcase, c->hcase, sizeof(CaseDev) * ncases, cudaMemcpyHostToDevice, c->stream));
   CKC(cudaMalloc(&c->dqueue, sizeof(int) * 10));
@@ -1186,15 +1140,10 @@ extern "C" int mbm_destroy(mbm_ctx* c) {
   cudaFree(c->dcfl);
   if (c->hcfl) cudaFreeHost(c->hcfl);
   if (c->ev) cudaEventDestroy(c->ev);
-  if (c->fork_ev) cudaEventDestroy(c->fork_ev);
   if (c->out_stream) cudaStreamSynchronize(c->out_stream);
   cudaFree(c->out_stage);
   if (c->out_ev) cudaEventDestroy(c->out_ev);
   if (c->out_stream) cudaStreamDestroy(c->out_stream);
-  for (int k = 0; k < 4; k++) {
-    if (c->join_ev[k]) cudaEventDestroy(c->join_ev[k]);
-    if (c->aux[k]) cudaStreamDestroy(c->aux[k]);
-  }
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return MBM_OK;
@@ -1489,8 +1438,7 @@ extern "C" int mbm_steps(mbm_ctx* c, double* t, double tend, double CFLmax, doub
 
 extern "C" int mbm_config(mbm_ctx* c, int* segment_rows, int* work_items, int* ctas) {
   if (!c) return fail(c, MBM_EINVAL, "mbm_config: null context");
-  int g = 0;
-  for (const LimGroup& x : c->groups[0]) g = std::max(g, std::max(x.grid[0], x.grid[1]));
+  const int g = std::max(c->grid[0], c->grid[1]);
   if (segment_rows) *segment_rows = (int)std::lround(c->seg_rows[0]);
   if (work_items) *work_items = c->nwork[0];
   if (ctas) *ctas = g;
@@ -1506,7 +1454,7 @@ extern "C" int mbm_bulk_copies(mbm_ctx* c, int* on) {
 
 extern "C" int mbm_dependent_launch(mbm_ctx* c, int* on) {
   if (!c || !on) return fail(c, MBM_EINVAL, "mbm_dependent_launch: bad argument");
-  *on = c->pdl && c->groups[0].size() <= 1 && c->groups[1].size() <= 1 ? 1 : 0;
+  *on = c->pdl ? 1 : 0;
   return MBM_OK;
 }
 
@@ -1518,8 +1466,7 @@ extern "C" int mbm_ghost_scatter(mbm_ctx* c, int* on) {
 
 extern "C" int mbm_config_stage(mbm_ctx* c, int heun, double* segment_rows, int* work_items, int* ctas) {
   if (!c || (heun != 0 && heun != 1)) return fail(c, MBM_EINVAL, "mbm_config_stage: bad argument");
-  int g = 0;
-  for (const LimGroup& x : c->groups[heun]) g = std::max(g, x.grid[heun]);
+  const int g = c->grid[heun];
   if (segment_rows) *segment_rows = c->seg_rows[heun];
   if (work_items) *work_items = c->nwork[heun];
   if (ctas) *ctas = g;
@@ -1674,7 +1621,7 @@ static int frozen_begin(mbm_ctx* c) {
 // consecutive steps queue without a host round trip)
 static int frozen_step(mbm_ctx* c, const double* in, double* out, const double* ddt, double* tmp) {
   double* bufs[3] = {const_cast<double*>(in), out, tmp};
-  PdlScope pdl_scope(c->pdl && c->groups[0].size() <= 1 && c->groups[1].size() <= 1);
+  PdlScope pdl_scope(c->pdl);
   CK(launch_frozen_prep(c->dcase, ddt, c->dqueue, c->stream));
   CK(launch_stages(c, 0, SEL_CUR, SEL_CUR, SEL_TMP, 0, bufs, true));
   if (!c->gscatter) CK(launch_ghost(c->dblk, c->dcase, c->dghost, c->nghost, bufs, c->ddir, SEL_TMP, c->stream));

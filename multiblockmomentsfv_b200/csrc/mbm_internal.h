@@ -27,11 +27,14 @@ constexpr int TILE_ROWS = 4;     // output rows of a tile (28 x 4 cells, mbm_til
 // two measured alike (a step of 4 x n^2 cells, harmonic, tiles / march in us):
 //   bitwise  n = 61: 23.6 / 51.3   192: 92 / 103   224 (2,052 tiles): 128 / 146   240: 144 / 145
 //   fast     n = 61: 14.6 / 33.3   192: 49 / 53    224: 68 / 68   256 (2,600 tiles): 97 / 78
-// Several limiters in a batch are as many launches for the march, none more for the tiles
-// (bitwise, 8 cases, 4,668 tiles: 318 / 359; 7,469: 482 / 488; fast, 2,567: 98 / 92).
-constexpr int TILE_MOST_EXACT = 2100, TILE_MOST_EXACT_BATCH = 7000, TILE_MOST_FAST = 1700;
+// A batch of several limiters costs the march more (its limiter is then taken at run time):
+//   bitwise  8 cases, 2,567 tiles: 159 / 172   4,668: 285 / 280;   fast  2,567: 88 / 83
+constexpr int TILE_MOST_EXACT = 2100, TILE_MOST_EXACT_BATCH = 4500, TILE_MOST_FAST = 1700;
 constexpr int CTA_WARPS = 4;     // warps per CTA of the persistent stage kernel
 constexpr int MAX_TRACE = 4096;  // progress records kept per case and Steps call
+
+// a stage launch over cases of several limiters: each block's own, at run time
+constexpr int LIM_ANY = 5;
 
 enum LayerSel : int { SEL_CUR = 0, SEL_OTHER = 1, SEL_TMP = 2 };
 

@@ -416,6 +416,25 @@ __device__ __forceinline__ double limit(double d1, double d2) {
 #endif
 }
 
+#if MBM_FAST_ARITH
+// S = Limit1(d1, d2) of N components by limiter LIM, or by lim if LIM is LIM_ANY
+template <int LIM, int N>
+__device__ __forceinline__ void limits(const double (&d1)[N], const double (&d2)[N], int lim, double (&S)[N]) {
+  if constexpr (LIM == LIM_ANY) {
+    switch (lim) {
+      case 0: limits<0>(d1, d2, lim, S); return;
+      case 1: limits<1>(d1, d2, lim, S); return;
+      case 2: limits<2>(d1, d2, lim, S); return;
+      case 3: limits<3>(d1, d2, lim, S); return;
+      default: limits<4>(d1, d2, lim, S); return;
+    }
+  } else {
+#pragma unroll
+    for (int n = 0; n < N; n++) S[n] = limit<LIM>(d1[n], d2[n]);
+  }
+}
+#endif
+
 #if !MBM_FAST_ARITH
 // L = Limit1(d1, d2) and the slope L / h of N components (src/Main.c:346-349), D =
 // Recip(h), h in the safe range.  The harmonic limiter's quotient has a denominator of its
@@ -454,6 +473,23 @@ __device__ __forceinline__ void slopes(const double (&d1)[N], const double (&d2)
   if (__builtin_expect(g.lo < (623u << 21) || g.hi >= (1424u << 21) || md >= (1103u << 20) || ones || D.bad, 0)) {
 #pragma unroll
     for (int n = 0; n < N; n++) S[n] = div_ieee(limit<LIM>(d1[n], d2[n]), D.y);
+  }
+}
+
+// the same by the limiter LIM, or by lim if LIM is LIM_ANY
+template <int LIM, int N>
+__device__ __forceinline__ void slopes_of(const double (&d1)[N], const double (&d2)[N], const Recip& D, int lim,
+                                          double (&S)[N]) {
+  if constexpr (LIM != LIM_ANY) {
+    slopes<LIM>(d1, d2, D, S);
+  } else {
+    switch (lim) {
+      case 0: slopes<0>(d1, d2, D, S); return;
+      case 1: slopes<1>(d1, d2, D, S); return;
+      case 2: slopes<2>(d1, d2, D, S); return;
+      case 3: slopes<3>(d1, d2, D, S); return;
+      default: slopes<4>(d1, d2, D, S); return;
+    }
   }
 }
 #endif

@@ -199,6 +199,7 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
   if (cs.done) return true;
   const int cur = cs.cur;
   const double dt = cs.dt, Fx = cs.F;
+  const int lim = cs.limiter;
   const Recip Kn(cs.Kn);
   const double* __restrict__ in = layer_ptr(a.buf, phys_layer(a.sel_in, cur)) + B.off;
   const double* __restrict__ d0 = layer_ptr(a.buf, phys_layer(a.sel_d0, cur)) + B.off;
@@ -374,10 +375,15 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
     if (r >= rs + 2) {
       double hi[NV], S[NV];
       // the face states P -+ (dy/2) (L/dy) are P -+ L/2: dy cancels
+      {
+        double d1[NV], d2[NV];
 #pragma unroll
-      for (int n = 0; n < NV; n++) {
-        const double pm = win.P[sm2][n][lane], p0 = win.P[sm1][n][lane], pp = win.P[s0][n][lane];
-        S[n] = limit<LIM>(p0 - pm, pp - p0);
+        for (int n = 0; n < NV; n++) {
+          const double p0 = win.P[sm1][n][lane];
+          d1[n] = p0 - win.P[sm2][n][lane];
+          d2[n] = win.P[s0][n][lane] - p0;
+        }
+        limits<LIM>(d1, d2, lim, S);
       }
 #pragma unroll
       for (int n = 0; n < NV; n++) {
@@ -414,11 +420,15 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
       __syncwarp();   // the window row is read across lanes below (other lanes wrote it)
       // the right-hand difference of a lane is its right neighbour's left-hand one (the
       // same subtraction of the same operands), passed down instead of recomputed
+      {
+        double d1[NV], d2[NV];
 #pragma unroll
-      for (int n = 0; n < NV; n++) {
-        P0[n] = win.P[sm2][n][lane];
-        const double d1 = P0[n] - win.P[sm2][n][(lane + 31) & 31];   // left neighbour (lane 0: unused)
-        Sx[n] = limit<LIM>(d1, __shfl_down_sync(0xffffffffu, d1, 1));
+        for (int n = 0; n < NV; n++) {
+          P0[n] = win.P[sm2][n][lane];
+          d1[n] = P0[n] - win.P[sm2][n][(lane + 31) & 31];   // left neighbour (lane 0: unused)
+          d2[n] = __shfl_down_sync(0xffffffffu, d1[n], 1);
+        }
+        limits<LIM>(d1, d2, lim, Sx);
       }
 #pragma unroll
       for (int n = 0; n < NV; n++) {        // P -+ L/2, as for the y faces
@@ -583,6 +593,7 @@ int stage_ctas_per_sm(int heun) {
     const unsigned long long bit = dev < 64 ? (1ull << dev) : 0ull;
     if (!bit || !(done & bit)) {
       smem_attr<0, 0>(); smem_attr<0, 1>(); smem_attr<0, 2>(); smem_attr<0, 3>(); smem_attr<0, 4>();
+      smem_attr<0, LIM_ANY>(); smem_attr<1, LIM_ANY>();
       smem_attr<1, 0>(); smem_attr<1, 1>(); smem_attr<1, 2>(); smem_attr<1, 3>(); smem_attr<1, 4>();
       done |= bit;
     }
@@ -604,6 +615,8 @@ static cudaError_t launch_stage_lim(int lim, const StageArgs& a, int grid, cudaS
     case 1: return launch_k(stage_kernel<HEUN, 1, TMA>, dim3(grid), dim3(32 * STAGE_WARPS), stage_smem<HEUN>(), s, a);
     case 2: return launch_k(stage_kernel<HEUN, 2, TMA>, dim3(grid), dim3(32 * STAGE_WARPS), stage_smem<HEUN>(), s, a);
     case 3: return launch_k(stage_kernel<HEUN, 3, TMA>, dim3(grid), dim3(32 * STAGE_WARPS), stage_smem<HEUN>(), s, a);
+    case LIM_ANY:
+      return launch_k(stage_kernel<HEUN, LIM_ANY, TMA>, dim3(grid), dim3(32 * STAGE_WARPS), stage_smem<HEUN>(), s, a);
     default: return launch_k(stage_kernel<HEUN, 4, TMA>, dim3(grid), dim3(32 * STAGE_WARPS), stage_smem<HEUN>(), s, a);
   }
 }

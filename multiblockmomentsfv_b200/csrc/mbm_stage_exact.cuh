@@ -49,6 +49,7 @@ __device__ __forceinline__ void exact_item(const StageArgs& a, const Work w, con
   if (cs.done) return;
   const int cur = cs.cur;
   const double dt = cs.dt, Fx = cs.F;
+  const int lim = cs.limiter;
   const Recip Kn(cs.Kn);
   const double* __restrict__ in = layer_ptr(a.buf, phys_layer(a.sel_in, cur)) + B.off;
   const double* __restrict__ d0 = layer_ptr(a.buf, phys_layer(a.sel_d0, cur)) + B.off;
@@ -173,7 +174,7 @@ __device__ __forceinline__ void exact_item(const StageArgs& a, const Work w, con
           d2[n] = pp[off[n]] - p0[n];
         }
         const double h = 0.5 * (y ? B.dy : B.dx);
-        slopes<LIM>(d1, d2, y ? rdy : rdx, S);
+        slopes_of<LIM>(d1, d2, y ? rdy : rdx, lim, S);
         double* const up = y ? &win.lo[r & 1][0][lane] : pl;
 #pragma unroll
         for (int n = 0; n < NV; n++) {
@@ -272,6 +273,7 @@ int stage_ctas_per_sm(int heun) {
     const unsigned long long bit = dev < 64 ? (1ull << dev) : 0ull;
     if (!bit || !(done & bit)) {
       exact_attr<0, 0>(); exact_attr<0, 1>(); exact_attr<0, 2>(); exact_attr<0, 3>(); exact_attr<0, 4>();
+      exact_attr<0, LIM_ANY>(); exact_attr<1, LIM_ANY>();
       exact_attr<1, 0>(); exact_attr<1, 1>(); exact_attr<1, 2>(); exact_attr<1, 3>(); exact_attr<1, 4>();
       done |= bit;
     }
@@ -292,6 +294,7 @@ static cudaError_t launch_exact(int lim, const StageArgs& a, int grid, cudaStrea
     case 1: return launch_k(stage_exact<HEUN, 1>, g, b, EXACT_SMEM, s, a);
     case 2: return launch_k(stage_exact<HEUN, 2>, g, b, EXACT_SMEM, s, a);
     case 3: return launch_k(stage_exact<HEUN, 3>, g, b, EXACT_SMEM, s, a);
+    case LIM_ANY: return launch_k(stage_exact<HEUN, LIM_ANY>, g, b, EXACT_SMEM, s, a);
     default: return launch_k(stage_exact<HEUN, 4>, g, b, EXACT_SMEM, s, a);
   }
 }
