@@ -1,0 +1,47 @@
+"""Uploads that pass through the context's page-locked ring: the caller's buffer is its own again
+when the call returns, more of them than the ring holds are no fewer, sizes on both sides of
+what goes through it, and restart payloads."""
+import numpy as np
+import pytest
+
+import helpers as H
+from multiblockmomentsfv_b200 import blockfile as bf, solver as sv
+
+pytestmark = pytest.mark.gpu
+
+
+def test_buffer_reuse_and_ring_wrap():
+    """30 blocks of 20 x 34 cells (37 KB) and one of 120 x 130 (1.2 MB), uploaded three times over
+    from one buffer that is overwritten at once: each block holds its own values."""
+    sizes = [(20, 34)] * 30 + [(120, 130)]
+    d = bf.Deck()
+    d.blocks = [bf.Block(k + 1, 0.0, 1.0, 0.0, 1.0, nx, ny, (0, 0, 0, 0)) for k, (nx, ny) in enumerate(sizes)]
+    rng = np.random.default_rng(0)
+    with sv.Solver(d) as s:
+        for _ in range(3):
+            want = [rng.standard_normal((b.nyp, b.nxp, 9)) for b in d.blocks]
+            buf = {sz: np.empty((sz[1] + 6, sz[0] + 6, 9)) for sz in set(sizes)}
+            for b, U in enumerate(want):
+                a = buf[sizes[b]]
+                a[...] = U
+                s.upload(0, b, a)
+                a[...] = np.nan
+            for b, U in enumerate(want):
+                H.assert_bitwise(s.download(0, b), U, f"block {b}")
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_payload_buffer_reuse(dtype):
+    d = bf.Deck()
+    d.blocks = [bf.Block(k + 1, 0.0, 1.0, 0.0, 1.0, 9 + 60 * (k % 2), 8, (0, 0, 0, 0)) for k in range(4)]
+    rng = np.random.default_rng(1)
+    with sv.Solver(d) as s:
+        want = []
+        for b, blk in enumerate(d.blocks):
+            p = (1 + rng.random(((blk.nx + 2) * (blk.ny + 2), 10))).astype(dtype)
+            s.load_fields(b, p, faithful=True)
+            want.append(s.download(0, b))
+            s.load_fields(b, p, faithful=True)
+            p[...] = 0
+        for b in range(4):
+            H.assert_bitwise(s.download(0, b), want[b], f"block {b}")
