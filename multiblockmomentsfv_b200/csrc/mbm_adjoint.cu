@@ -223,13 +223,18 @@ __device__ __forceinline__ void data0_adj(const AdjArgs& a, const BlockDev& B, i
 }
 
 // the rest of a cell's share once its reconstruction and slope adjoints Pb are gathered;
-// D0: the Data0 term here too (stage 2 of the fused cell pass)
+// D0: the Data0 term here too (stage 2 of the fused cell pass).  All of the cell's values are
+// asked for before any arithmetic: one wait for memory, not one per layer.
 template <int HEUN, bool D0>
 __device__ __forceinline__ double cell_rest(const AdjArgs& a, const BlockDev& B, int I, int J,
                                             const double (&Pb)[NV]) {
-  double Ub[NV] = {0}, U[NV], P0[NV];
+  const long long ic = cidx(B, I, J);
+  const bool upd = inner(B, I, J);
+  double Ub[NV] = {0}, U[NV], P0[NV], Rb[NV], X[NV];
   double knb = 0.0;
   load9(a.x, B, I, J, U);
+  if (upd) load9(a.lout, B, I, J, Rb);
+  if (!HEUN) load9(a.lx, B, I, J, X);
   mbm_adj::prim(U, P0);
   double Qb[NV] = {0};
   bool anyP = false;
@@ -238,14 +243,13 @@ __device__ __forceinline__ double cell_rest(const AdjArgs& a, const BlockDev& B,
   if (anyP) {     // Aux = relax(Primitive(U), 2H+1) off the ring (ring cells never reach a face)
     mbm_adj::relax_p_adj(P0, Pb, Qb, &knb, a.dt, a.Kn, 2 * HEUN + 1);
   }
-  const long long ic = cidx(B, I, J);
   double Vb[NV] = {0};
-  if (inner(B, I, J)) {
+  if (upd) {
     // update term R: Conservative(relax(Primitive(X), 2H)) [+ Conservative(relax(Primitive(D0), -1))]
     const double s = HEUN ? 0.5 : 1.0;
-    double Rb[NV], Q[NV], Cb[NV] = {0};
+    double Q[NV], Cb[NV] = {0};
 #pragma unroll
-    for (int m = 0; m < NV; m++) Rb[m] = s * a.lout[cidx(B, I, J) + m * B.plane];
+    for (int m = 0; m < NV; m++) Rb[m] = s * Rb[m];
     mbm_adj::relax_p(P0, Q, a.dt, a.Kn, a.F, 2 * HEUN);
     mbm_adj::cons_adj(Q, Rb, Cb);
     mbm_adj::relax_p_adj(P0, Cb, Qb, &knb, a.dt, a.Kn, 2 * HEUN);
@@ -265,7 +269,7 @@ __device__ __forceinline__ double cell_rest(const AdjArgs& a, const BlockDev& B,
     }
   } else if (anyQ) {
 #pragma unroll
-    for (int m = 0; m < NV; m++) a.lx[ic + m * B.plane] += Ub[m];
+    for (int m = 0; m < NV; m++) a.lx[ic + m * B.plane] = X[m] + Ub[m];
   }
   return knb;
 }
@@ -305,8 +309,8 @@ __global__ void __launch_bounds__(128, ADJ_CELL_CTAS) adj_cells(AdjArgs a, long 
 // and spilled them (about 80 MB of DRAM writes per launch at 4 x 256^2).  The Data0 term,
 // a function of Data0 and the output adjoint alone, moves to the primitives pass of stage
 // 2; the gather of the reconstruction and slope adjoints (the neighbour loads) stores Pb;
-// a pointwise pass takes it through the relaxation and Primitive.  The same operations
-// in the same order per cell; only dJ/dKn's atomic sums are grouped differently.
+// a pointwise pass takes it through the relaxation and Primitive.  The same terms
+// per cell, the gathered ones added in another order, and dJ/dKn's atomic sums grouped otherwise.
 
 // pass A of stage 2 with the Data0 term: the projected primitives as adj_prims, and the
 // Data0 adjoint of every cell (zero off the interior), which starts that adjoint layer
@@ -340,35 +344,109 @@ __global__ void adj_prims_d0(AdjArgs a, long long nthr) {
   if ((threadIdx.x & 31) == 0 && knb != 0.0) atomicAdd(a.knb, knb);
 }
 
-// pass C1: the reconstruction and slope adjoints Pb of every cell (zero on the ring)
+// pass C1: the reconstruction and slope adjoints Pb of every cell off the ring.  A warp marches
+// one component up a strip of 28 columns (32 lanes with a halo of 2 on each side) and a
+// segment of GROWS rows: a cell's limiter derivatives along x and along y are formed once and
+// handed to its neighbours, through shuffles along x and from row to row along y -- as a
+// thread per cell, which read its neighbourhood and formed the derivatives of its neighbours
+// as well, the pass took 21 loads, six derivatives and 108 instructions a cell instead of 5,
+// 2.3 and 83, and 55 us at 4 x 256^2 instead of 39 (harmonic).  What is left are the limiter's
+// derivatives.  Clamped rows and columns in place of the predicated loads, with 32-bit offsets,
+// took more registers and 52 us; GROWS 24 and 32 were no faster than 16.
+constexpr int GWARPS = 4;
+
+// l * dL/dd1 / h and l * dL/dd2 / h of a cell with slope adjoint l / (h/2) = d, and their
+// difference; nothing where l is zero (cells no output depends on may hold no state, and
+// 0 * NaN would leak into the sum)
 template <int LIM>
-__global__ void __launch_bounds__(128, ADJ_CELL_CTAS) adj_gather(AdjArgs a, long long nthr, const double* FLx,
-                                                     const double* FRx, const double* FLy, const double* FRy) {
+__device__ __forceinline__ void slope_adj(double d, double h, double rh, double d1, double d2, bool on, double& ga,
+                                          double& gb, double& gd) {
+  const double l = 0.5 * h * d;
+  ga = gb = gd = 0.0;
+  if (on && l != 0.0) {
+    double g1, g2;
+    mbm_adj::limit_grad(LIM, d1, d2, &g1, &g2);
+    ga = l * g1 * rh;
+    gb = l * g2 * rh;
+    gd = l * (g1 - g2) * rh;
+  }
+}
+
+template <int LIM>
+__global__ void __launch_bounds__(32 * GWARPS) adj_gather(AdjArgs a, const double* __restrict__ FLx,
+                                                           const double* __restrict__ FRx, const double* __restrict__ FLy,
+                                                           const double* __restrict__ FRy) {
   pdl_enter();
-  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  int b, I, J;
-  if (k >= nthr || !locate(a.blk, a.nblk, k, b, I, J)) return;
+  const int lane = threadIdx.x & 31, m = blockIdx.y;
+  long long item = (long long)blockIdx.x * GWARPS + (threadIdx.x >> 5);
+  int b = 0;
+  for (; b < a.nblk; b++) {
+    const long long n = gather_items(a.blk[b].nxp, a.blk[b].nyp);
+    if (item < n) break;
+    item -= n;
+  }
+  if (b == a.nblk) return;
   const BlockDev B = a.blk[b];
-  const bool ring = I == 0 || J == 0 || I == B.nxp - 1 || J == B.nyp - 1;
-  const long long i0 = cidx(B, I, J);
-#pragma unroll 1
-  for (int m = 0; m < NV; m++) {        // (0 + x term) + y term, as the whole pass sums them
-    const long long i = i0 + m * B.plane;
-    double v = 0.0;
-    if (!ring) {
-      v += gather_comp<LIM>(a, B, I, J, 1, FLx, FRx, i);
-      v += gather_comp<LIM>(a, B, I, J, 2, FLy, FRy, i);
+  const int nxp = B.nxp, nyp = B.nyp, pitch = B.pitch;
+  const int strips = (nxp - 2 + STRIP - 1) / STRIP;
+  const int sg = (int)(item / strips), st = (int)(item - (long long)sg * strips);
+  const int C = 1 + st * STRIP - 2 + lane;
+  const int J0 = 1 + sg * GROWS, J1 = min(J0 + GROWS, nyp - 1);        // output rows [J0, J1)
+  const bool in = C >= 0 && C < nxp, out = lane >= 2 && lane <= 29 && C <= nxp - 2;
+  const bool xs = C >= 1 && C <= nxp - 2;                               // off the ring along x
+  const double rhx = mbm_adj::rcp(B.dx), rhy = mbm_adj::rcp(B.dy);
+  const long long base = B.off + m * B.plane + C + 1;
+  const double* P = a.P + base;
+  auto at = [&](const double* p, int J) -> double {      // row J of this lane's column (0 off the block)
+    return in && J >= 0 && J < nyp ? p[(long long)J * pitch] : 0.0;
+  };
+  FLx += base; FRx += base; FLy += base; FRy += base;
+  // rows k-1, k, k+1 of P; the adjoints of the y faces above and below row k; the derivatives
+  // of rows k-1 and k-2
+  double pm = at(P, J0 - 2), p0 = at(P, J0 - 1), frm = at(FRy, J0 - 2), flm = 0.0, frmm = 0.0;
+  double gbm = 0.0, gdm = 0.0, gbmm = 0.0;
+  double pp = at(P, J0), fl = at(FLy, J0 - 1), fr = at(FRy, J0 - 1), fx = 0.0, rx = 0.0;
+  for (int k = J0 - 1; k <= J1; k++) {
+    // the next row's values on their way
+    const double ppn = at(P, k + 2), fln = at(FLy, k + 1), frn = at(FRy, k + 1);
+    const double fxn = at(FLx, k), rxn = at(FRx, k);
+    double ga, gb, gd;
+    slope_adj<LIM>(fl - frm, B.dy, rhy, p0 - pm, pp - p0, k >= 1 && k <= nyp - 2, ga, gb, gd);
+    if (k > J0) {           // output row k-1: its x terms, then the y terms
+      // left state of face c|c+1, right state of face c-1|c; S(q) = L(P(q)-P(q-1), P(q+1)-P(q)) / h
+      const double p = pm, rxm = __shfl_up_sync(0xffffffffu, rx, 1);
+      const double pl = __shfl_up_sync(0xffffffffu, p, 1), pr = __shfl_down_sync(0xffffffffu, p, 1);
+      double xa, xb, xd;
+      slope_adj<LIM>(fx - rxm, B.dx, rhx, p - pl, pr - p, xs, xa, xb, xd);
+      const double xbl = __shfl_up_sync(0xffffffffu, xb, 1), xar = __shfl_down_sync(0xffffffffu, xa, 1);
+      const double gx = ((fx + rxm) + xd) + xbl - xar;
+      const double gy = ((flm + frmm) + gdm) + gbmm - ga;
+      if (out) a.Pb[base + (long long)(k - 1) * pitch] = gx + gy;
     }
-    a.Pb[i] = v;
+    gbmm = gbm;
+    gbm = gb;
+    gdm = gd;
+    frmm = frm;
+    flm = fl;
+    pm = p0;
+    p0 = pp;
+    pp = ppn;
+    frm = fr;
+    fl = fln;
+    fr = frn;
+    fx = fxn;
+    rx = rxn;
   }
 }
 
 // pass C2: per cell, Pb through the relaxation and Primitive to the stage input, with the
 // update's relaxation term (the Data0 term is in pass A)
 #ifndef ADJ_POINT_CTAS
-// resident 128-thread CTAs per SM the pointwise pass is compiled for: 6 (80 registers, 64
-// bytes of spills) ran the reverse sweep 1 ms faster than 4 (no spills), 5 or 8 (4 x 256^2)
-#define ADJ_POINT_CTAS 6
+// resident 128-thread CTAs per SM the pointwise pass is compiled for: a cell's loads are all
+// asked for at the start, so four without spills keep enough of them in flight and ran the
+// reverse sweep of 60 steps at 4 x 256^2 in 18.0 ms, six (64 bytes of spills) in 18.3.  The
+// pass takes 26 us; with the loads of a layer asked for where it is used it took 36.
+#define ADJ_POINT_CTAS 4
 #endif
 template <int HEUN>
 __global__ void __launch_bounds__(128, ADJ_POINT_CTAS) adj_point(AdjArgs a, long long nthr) {
@@ -379,9 +457,10 @@ __global__ void __launch_bounds__(128, ADJ_POINT_CTAS) adj_point(AdjArgs a, long
   if (k < nthr && locate(a.blk, a.nblk, k, b, I, J)) {
     const BlockDev B = a.blk[b];
     const long long i = cidx(B, I, J);
+    const bool ring = I == 0 || J == 0 || I == B.nxp - 1 || J == B.nyp - 1;
     double Pb[NV];
 #pragma unroll
-    for (int m = 0; m < NV; m++) Pb[m] = a.Pb[i + m * B.plane];
+    for (int m = 0; m < NV; m++) Pb[m] = ring ? 0.0 : a.Pb[i + m * B.plane];
     knb = cell_rest<HEUN, false>(a, B, I, J, Pb);
   }
 #pragma unroll
@@ -389,24 +468,30 @@ __global__ void __launch_bounds__(128, ADJ_POINT_CTAS) adj_point(AdjArgs a, long
   if ((threadIdx.x & 31) == 0 && knb != 0.0) atomicAdd(a.knb, knb);
 }
 
-// adjoint of the ghost fill: ghost adjoint -> its source cell (wall signs), then
-// zero; one thread per (ghost cell, component)
-__global__ void adj_ghosts(const BlockDev* __restrict__ blk, const GhostEntry* __restrict__ map, int n, double* l) {
+// adjoint of the ghost fill: ghost adjoint -> its source cell (wall signs), then zero; one
+// thread per ghost cell, its nine components in flight together (a thread per component,
+// neighbouring threads in different planes, took 15 us at 4 x 256^2, 7 like this)
+__global__ void __launch_bounds__(128) adj_ghosts(const BlockDev* __restrict__ blk, const GhostEntry* __restrict__ map,
+                                                  int n, double* l) {
   pdl_enter();
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)n * NV) return;
-  const int i = (int)(t / NV), m = (int)(t - (long long)i * NV);
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
   const GhostEntry e = map[i];
-  const BlockDev D = blk[e.dst_blk];
-  double* g = l + D.off + e.dst + m * D.plane;
-  const double v = *g;
-  *g = 0.0;
-  if (e.src < 0 || v == 0.0) return;          // Dirichlet ghosts have no source
-  const int sblk = e.src_blk_flags & 0xffff;
+  const BlockDev D = blk[e.dst_blk], S = blk[e.src < 0 ? 0 : e.src_blk_flags & 0xffff];
+  double* g = l + D.off + e.dst;
+  double v[NV];
+#pragma unroll
+  for (int m = 0; m < NV; m++) v[m] = g[m * D.plane];
+#pragma unroll
+  for (int m = 0; m < NV; m++) g[m * D.plane] = 0.0;
+  if (e.src < 0) return;          // Dirichlet ghosts have no source
   const bool fx = (e.src_blk_flags >> 16) & 1, fy = (e.src_blk_flags >> 17) & 1;
-  const BlockDev S = blk[sblk];
-  const bool flip = (fx && (m == 1 || m == 5 || m == 7)) != (fy && (m == 2 || m == 5 || m == 8));
-  atomicAdd(l + S.off + e.src + m * S.plane, flip ? -v : v);
+  double* s = l + S.off + e.src;
+#pragma unroll
+  for (int m = 0; m < NV; m++) {
+    const bool flip = (fx && (m == 1 || m == 5 || m == 7)) != (fy && (m == 2 || m == 5 || m == 8));
+    if (v[m] != 0.0) atomicAdd(s + m * S.plane, flip ? -v[m] : v[m]);
+  }
 }
 
 // J = sum over interior cells of f(P) of the final state, and dJ/dU; f by `kind`:
@@ -738,8 +823,8 @@ static void faces_cells(const AdjArgs& a0, long long nthr, unsigned G, double* F
                         double* FRy, cudaStream_t s) {
   launch_k(adj_faces<HEUN, LIM>, dim3(G), dim3(128), 0, s, a0, nthr, FLx, FRx, FLy, FRy);
   if (a0.Pb) {
-    launch_k(adj_gather<LIM>, dim3(G), dim3(128), 0, s, a0, nthr, (const double*)FLx, (const double*)FRx,
-             (const double*)FLy, (const double*)FRy);
+    launch_k(adj_gather<LIM>, dim3((unsigned)((a0.ngather + GWARPS - 1) / GWARPS), NV), dim3(32 * GWARPS), 0, s, a0,
+             (const double*)FLx, (const double*)FRx, (const double*)FLy, (const double*)FRy);
     launch_k(adj_point<HEUN>, dim3(G), dim3(128), 0, s, a0, nthr);
   } else {
     launch_k(adj_cells<HEUN, LIM>, dim3(G), dim3(128), 0, s, a0, nthr, (const double*)FLx, (const double*)FRx,
@@ -774,7 +859,7 @@ cudaError_t adjoint_stage(const AdjArgs& a0, long long nthr, double* FLx, double
 
 cudaError_t adjoint_ghosts(const BlockDev* blk, const GhostEntry* map, int n, double* l, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  launch_k(adj_ghosts, dim3((unsigned)(((long long)n * NV + 255) / 256)), dim3(256), 0, s, blk, map, n, l);
+  launch_k(adj_ghosts, dim3((unsigned)((n + 127) / 128)), dim3(128), 0, s, blk, map, n, l);
   return cudaGetLastError();
 }
 

@@ -1693,6 +1693,7 @@ static int adj_step(mbm_ctx* c, const double* Dn, const double* Tn, double dt, d
   a.work = c->adj_work;
   a.nwork = c->adj_nwork;
   a.queue = c->adj_queue;
+  for (auto& d : c->hblk) a.ngather += gather_items(d.nxp, d.nyp);
   a.blk = c->dblk;
   a.nblk = c->nblk;
   a.P = P;

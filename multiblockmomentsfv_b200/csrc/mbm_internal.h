@@ -158,7 +158,15 @@ struct AdjArgs {       // one stage of the discrete adjoint (mbm_adjoint.cu)
   const Work* work;      // row-marching pass: strips of ASTRIP columns x row segments
   int nwork;
   int* queue;            // its work-item counter (zero before the launch)
+  long long ngather;     // work items of the gather per component
 };
+
+// work items (warps) of the adjoint's gather for one component of a block: strips of STRIP columns
+// x segments of GROWS rows of the cells off the ring
+constexpr int GROWS = 16;
+__host__ __device__ inline long long gather_items(int nxp, int nyp) {
+  return (long long)((nxp - 2 + STRIP - 1) / STRIP) * ((nyp - 2 + GROWS - 1) / GROWS);
+}
 
 constexpr int ASTRIP = 26;   // output columns of one warp of the row-marching adjoint
 
