@@ -105,19 +105,21 @@ __device__ __forceinline__ void scatter_item(const StageArgs& a, int wi, int lan
 #if MBM_FAST_ARITH
 // Rolling state of one warp, lane fastest (conflict-free 8-byte accesses): the
 // projected primitives of three consecutive rows, the lower state of the next
-// y face and the y flux of the face below the row being finished.  Stage 2 adds two
-// slots its asynchronous copies land in (stage 1 prefetches into registers).  Measured
-// and dropped: stage 1 keeping its relaxation terms in a window ring instead of reading
-// them back from global memory (neutral to 5 % slower), and stage 2 copying the update
-// row's moments into a third slot (per-lane copies: 20 % slower than loading them).
+// y face and the y flux of the face below the row being finished, and the slots the
+// asynchronous copies of what the next row's update needs land in.  Measured and dropped:
+// stage 1 keeping its relaxation terms in a ring of three rows instead of copying them
+// back from global memory (neutral to 5 % slower), and stage 2 copying the next row's
+// moments as well as the update row's into slots (20 % slower: the shared memory comes
+// out of L1; the next row's are in registers).
 struct WarpWindow1 {
   double P[3][NV][32];
   double lo[NV][32];
   double G[NV][32];
+  double D0a[NV][32];     // stage 1: the relaxation term of the next update row; stage 2: Data0,
+                          // or its stored relaxation term, of that row
 };
 struct WarpWindow2 : WarpWindow1 {
-  double Ua[NV][32];      // the moments of the next row
-  double D0a[NV][32];     // Data0 (or its stored relaxation term) of the next update row
+  double Ua[NV][32];      // the moments of the next update row (bulk copies: of the next row)
   // completion barriers of the bulk tensor copies into Ua and into D0a; the padding
   // keeps every slot of every warp's window on a 128-byte boundary
   unsigned long long bar[2];
@@ -205,11 +207,11 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
   const double* __restrict__ d0 = layer_ptr(a.buf, phys_layer(a.sel_d0, cur)) + B.off;
   double* __restrict__ out = layer_ptr(a.buf, phys_layer(a.sel_out, cur)) + B.off;
   // the relaxation term of the stage-1 input (flag -1): written by stage 1 at its row r,
-  // read back, with plain loads, by the update of that row two iterations later; stage 2
-  // reads it with rlx_read in place of forming it from Data0
-  double* __restrict__ rlx = a.rlx ? a.rlx + B.off : nullptr;
+  // copied back by the same thread in time for the update of that row two iterations later;
+  // stage 2 reads it with rlx_read in place of forming it from Data0
+  double* rlx = a.rlx ? a.rlx + B.off : nullptr;      // stage 1 also copies from it: no __restrict__
   const bool rlx_rd = HEUN == 1 && a.rlx_read;
-  const double* __restrict__ d0src = rlx_rd ? rlx : d0;
+  const double* const d0src = HEUN == 0 || rlx_rd ? rlx : d0;
   const int nxp = B.nxp, nyp = B.nyp, pitch = B.pitch;
   const long long plane = B.plane;
   const int C = w.I0 - 2 + lane;
@@ -227,14 +229,18 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
   // and the y face (r-2 | r-1), then finishes row J = r-2 (x face, update).
   const int rs = w.J0 >= 2 ? w.J0 - 2 : w.J0 - 1;
   int s0 = rs % 3;                 // window slot of row r
-  // Stage 1 loads the moments of row r+1 while it works on row r (nine registers,
-  // which stage 2, holding Data0 as well, cannot spare without spilling).
-  constexpr bool PREFETCH = HEUN == 0;
-  // Stage 2 copies, without registers, the moments of row r+1 into shared memory while
-  // it works on row r, and Data0 (or its relaxation term) of update row J+1 while it
-  // finishes row J (= r-2):
-  // one group per fetch, committed even when empty, so that the groups alternate
-  // U(r), D0(r-2), U(r+1), D0(r-1), ... and each wait leaves only the newest in flight
+  // The moments of row r+1 are loaded while row r is worked on, as soon as row r's have been
+  // used (the same nine registers).  What the update of row J+1 needs from memory -- stage 1:
+  // its relaxation term; stage 2: its moments, and Data0 or its relaxation term -- is copied to
+  // shared memory, without registers, while row J (= r-2) ... J+1 are worked on: loaded where
+  // it is used, it was the longest wait of a row (the second longest in stage 2).  4 x 256^2 /
+  // 512^2 / 1024^2 cells, harmonic: stage 1 34.9 / 99.9 / 333 -> 33.3 / 96.3 / 329 us, stage 2
+  // 34.8 / 98.5 / 320 -> 32.9 / 92.2 / 312 us; a step of 1024^2 666 -> 642 us.
+  constexpr bool PREFETCH = !TMA;
+  // With bulk copies, the moments of row r+1 go to shared memory as well, and those of row J
+  // are loaded again.  Where the window is not aligned for them, per-lane copies: one group per
+  // fetch, committed even when empty, so that the groups alternate U(r), D0(r-2), U(r+1),
+  // D0(r-1), ... and each wait leaves only the newest in flight.
   // bulk tensor copies: lane 0 issues each fetch after every lane has read the slot
   // (__syncwarp, then the proxy fence); a fetch of a row outside the block completes
   // its barrier phase with a plain arrive, so every fetch is matched by one wait
@@ -292,22 +298,23 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
         }
         return;
       }
-      if (col_out && Jn >= NG && Jn <= nyp - 1 - NG && Jn >= w.J0 && Jn < w.J1) {
-        const long long idx = (long long)Jn * pitch + C + 1;
-#pragma unroll
-        for (int n = 0; n < NV; n++) cp_async8(&win.D0a[n][lane], d0src + n * plane + idx);
-      }
-      cp_async_commit();
     }
+    if (col_out && Jn >= NG && Jn <= nyp - 1 - NG && Jn >= w.J0 && Jn < w.J1) {
+      const long long idx = (long long)Jn * pitch + C + 1;
+#pragma unroll
+      for (int n = 0; n < NV; n++) cp_async8(&win.D0a[n][lane], d0src + n * plane + idx);
+      if constexpr (HEUN == 1 && !TMA) {
+#pragma unroll
+        for (int n = 0; n < NV; n++) cp_async8(&win.Ua[n][lane], in + n * plane + idx);
+      }
+    }
+    cp_async_commit();
   };
   u_fetch(rs);
   d0_fetch(rs - 2);
   double Un[NV];
-  if (PREFETCH) {
-    const bool ok = col_in && rs >= 0 && rs < nyp;
-    if (ok) load_cell(in, plane, (long long)rs * pitch + C + 1, Un);
-    else benign(Un);
-  }
+  const int Cin = min(max(C, 0), nxp - 1);   // lanes and rows outside the grid: the nearest cell's values, unused
+  if (PREFETCH) load_cell(in, plane, (long long)rs * pitch + Cin + 1, Un);
   for (int r = rs; r <= w.J1 + 1; r++) {
     const int sm1 = s0 == 0 ? 2 : s0 - 1, sm2 = sm1 == 0 ? 2 : sm1 - 1;
     // (a) projected primitives of row r: Aux.Prim (src/Main.c:314-336)
@@ -317,10 +324,7 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
       if (PREFETCH) {
 #pragma unroll
         for (int n = 0; n < NV; n++) U[n] = Un[n];
-        const bool okn = col_in && r + 1 >= 0 && r + 1 < nyp;
-        if (okn) load_cell(in, plane, (long long)(r + 1) * pitch + C + 1, Un);
-        else benign(Un);
-      } else if constexpr (HEUN == 1) {
+      } else if constexpr (TMA) {
         if (tma) {
           if (!bar_wait(0)) { aborted = true; break; }
         } else {
@@ -335,6 +339,7 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
         u_fetch(r + 1);                      // into the slot just read
       }
       primitive(U, Q);
+      if (PREFETCH) load_cell(in, plane, (long long)min(r + 1, nyp - 1) * pitch + Cin + 1, Un);
       if (HEUN == 0) {
         // stage 1: one collision number and one reciprocal per damping argument serve
         // the CFL share (flag 0), the relaxation term of the update (flag -1, stored for
@@ -408,12 +413,12 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
     }
     // (c) row J = r-2: x slope, x face C | C+1 (src/Main.c:346-347, 372-378), update
     const int J = r - 2;
-    if (HEUN == 1) {                        // this row's Data0 and moments have landed
-      if (tma) {
-        if (!bar_wait(1)) { aborted = true; break; }
-      } else {
-        cp_async_wait_one();
-      }
+    if (tma) {                              // what this row's update needs has landed
+      if (!bar_wait(1)) { aborted = true; break; }
+    } else if (TMA) {
+      cp_async_wait_one();
+    } else {
+      cp_async_wait_all();
     }
     if (J >= w.J0 && J < w.J1) {
       double P0[NV], Sx[NV], lo[NV], hi[NV], F[NV];
@@ -449,11 +454,14 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
         const long long idx = (long long)J * pitch + C + 1;
         double U[NV], Q[NV], R[NV];
         const double g = dt * Fx;
-        if constexpr (HEUN == 1) {
+        if constexpr (TMA) {
           load_cell(in, plane, idx, U);
+        } else if constexpr (HEUN == 1) {
+#pragma unroll
+          for (int n = 0; n < NV; n++) U[n] = win.Ua[n][lane];
         } else {
 #pragma unroll
-          for (int n = 0; n < NV; n++) U[n] = rlx[n * plane + idx];   // relax<-1> of this cell
+          for (int n = 0; n < NV; n++) U[n] = win.D0a[n][lane];   // relax<-1> of this cell
         }
         // stage 1: relax<0> = the force push of relax<-1>; stage 2: relax<2> = the force
         // push of the moments (both the identity without a force)
@@ -493,7 +501,7 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
     d0_fetch(r - 1);                        // the next update row, into the slot row J has left
     s0 = s0 == 2 ? 0 : s0 + 1;
   }
-  if constexpr (HEUN == 1) {                // nothing in flight past the work item
+  if constexpr (TMA) {                      // nothing in flight past the work item
     if (tma) {
       if (aborted) {
         // a copy did not land within the bound: flag the case, give the copies still in
@@ -510,10 +518,9 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
         if (lane == 0) atomicOr(&a.cases[B.case_id].nonfinite, 2);
         return false;
       }
-    } else {
-      cp_async_wait_all();
     }
   }
+  if (!tma) cp_async_wait_all();
   if (a.gs_item) scatter_item(a, wi, lane, out - B.off, out, plane);
 
   stage_maxima<HEUN>(a, w.blk, B.case_id, lane, lamx, lamy, prod, expmax);
