@@ -97,10 +97,11 @@ struct mbm_ctx {
   std::string tma_note;             // why the stage-2 bulk tensor copies are off, if they are
   int* dtma_drop = nullptr;         // failure-detection test: device flag, the next bulk-copy launch withholds one copy
   double* staging = nullptr;        // array-of-structs transfer buffer, one block
-  // page-locked memory that small host inputs pass through, read there by the device; filled
-  // from the front until the next wait for the stream finds all of it consumed
+  // page-locked memory: first what small host inputs pass through, read there by the device,
+  // filled from the front until the next wait for the stream finds all of it consumed; then
+  // hcase, hcfl and hsync
   char* ring = nullptr;
-  size_t ring_used = 0;
+  size_t ring_used = 0, ring_bytes = 0;
   GhostEntry* dghost = nullptr;
   int nghost = 0;
   int* dgoff = nullptr;             // per block, its first entry of dghost
@@ -239,16 +240,11 @@ static int wait_stream(mbm_ctx* c) {
 // where the stream's kernels and copies read them: the call needs no wait for the device
 // before the caller may have its buffer back.  Null: too large, or no room to be had.
 // 28 uploads of 40 KB: 559 -> 275 us; the set-up of a Steps call or a ghost fill: 26 -> 16 us.
-constexpr size_t RING_BYTES = 1 << 20, RING_MOST = 256 << 10;
+constexpr size_t RING_BYTES = 440 << 10, RING_MOST = 256 << 10, RING_RECORDS = 16 << 10;
 
 static void* ring_put(mbm_ctx* c, const void* src, size_t bytes) {
-  if (bytes > RING_MOST) return nullptr;
-  if (!c->ring && cudaMallocHost((void**)&c->ring, RING_BYTES) != cudaSuccess) {
-    cudaGetLastError();
-    c->ring = nullptr;
-    return nullptr;
-  }
-  if (c->ring_used + bytes > RING_BYTES && wait_stream(c) != MBM_OK) return nullptr;   // empties it
+  if (bytes > RING_MOST || bytes > c->ring_bytes) return nullptr;
+  if (c->ring_used + bytes > c->ring_bytes && wait_stream(c) != MBM_OK) return nullptr;   // empties it
   void* p = c->ring + c->ring_used;
   memcpy(p, src, bytes);
   c->ring_used += (bytes + 255) & ~(size_t)255;
@@ -980,7 +976,23 @@ static int create_impl(const std::vector<mbm_block_desc>& glob, const std::vecto
 
   // controllers, maxima, queues, trace, per-block CFL
   CKC(cudaMalloc(&c->dcase, sizeof(CaseDev) * ncases));
-  CKC(cudaMallocHost(&c->hcase, sizeof(CaseDev) * ncases));
+  {
+    // all of the context's page-locked memory in one piece of less than 512 KB (unless the cases
+    // are many), the ring first: a context pays at most one page-locking of fresh memory, 0.8-2.6
+    // ms whatever its size, and contexts that live side by side share it.  Without a block whose
+    // state fits the ring, it takes case records only.
+    auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
+    c->ring_bytes = RING_RECORDS;
+    for (const auto& d : c->hblk)
+      if ((size_t)d.nxp * d.nyp * NV * sizeof(double) <= RING_MOST) c->ring_bytes = RING_BYTES;
+    const size_t cases_at = c->ring_bytes, cfl_at = cases_at + up(sizeof(CaseDev) * ncases);
+    const size_t sync_at = cfl_at + up(sizeof(double) * nblocks);
+    CKC(cudaMallocHost(&c->ring, sync_at + sizeof(unsigned)));
+    c->hcase = (CaseDev*)(c->ring + cases_at);
+    c->hcfl = (double*)(c->ring + cfl_at);
+    c->hsync = (unsigned*)(c->ring + sync_at);
+    *c->hsync = 0;
+  }
   memset(c->hcase, 0, sizeof(CaseDev) * ncases);
   for (int k = 0; k < ncases; k++) {
     CaseDev& h = c->hcase[k];
@@ -1001,7 +1013,6 @@ static int create_impl(const std::vector<mbm_block_desc>& glob, const std::vecto
   CKC(cudaMemsetAsync(c->dlam, 0, sizeof(unsigned long long) * 6 * nblocks, c->stream));
   CKC(cudaMalloc(&c->dtrace, sizeof(double) * 4 * MAX_TRACE * ncases));
   CKC(cudaMalloc(&c->dcfl, sizeof(double) * nblocks));
-  CKC(cudaMallocHost(&c->hcfl, sizeof(double) * nblocks));
 
   // work table and grid
   CKC(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device));
@@ -1020,8 +1031,6 @@ static int create_impl(const std::vector<mbm_block_desc>& glob, const std::vecto
     c->tile_grid = (int)std::min<long long>(tiles, (long long)c->nsm * tile_ctas);
     c->tile_loop = !c->adjoint && !shard && tiles <= (long long)TILE_MAX * c->tile_grid;
     CKC(cudaMalloc(&c->dsync, tile_scratch(c)));
-    CKC(cudaMallocHost(&c->hsync, sizeof(unsigned)));
-    *c->hsync = 0;
   }
   c->max_items = std::max<long long>(1, max_items);
   CKC(cudaMalloc(&c->dwork, sizeof(Work) * 2 * c->max_items));
@@ -1143,9 +1152,7 @@ extern "C" int mbm_destroy(mbm_ctx* c) {
   cudaFree(c->dgs_item);
   cudaFree(c->dwork);
   cudaFree(c->dsync);
-  if (c->hsync) cudaFreeHost(c->hsync);
   cudaFree(c->dcase);
-  if (c->hcase) cudaFreeHost(c->hcase);
   cudaFree(c->dlam);
   cudaFree(c->dqueue);
   for (int k = 0; k < 9; k++) cudaFree(c->adj_buf[k]);
@@ -1170,7 +1177,6 @@ extern "C" int mbm_destroy(mbm_ctx* c) {
   cudaFree(c->shard_cfl);
   cudaFree(c->dtrace);
   cudaFree(c->dcfl);
-  if (c->hcfl) cudaFreeHost(c->hcfl);
   if (c->ev) cudaEventDestroy(c->ev);
   if (c->out_stream) cudaStreamSynchronize(c->out_stream);
   cudaFree(c->out_stage);
