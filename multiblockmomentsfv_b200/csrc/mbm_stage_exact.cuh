@@ -11,11 +11,13 @@
 // instructions, more than an SM keeps close: its warps waited for instructions a fifth of the
 // time.  So the two directions are one loop, x and y swapped in the y pass (hll_swapped).  The
 // moments of the next row and Data0 of the row to be updated are copied to shared memory
-// while a row is worked on, and the update's other term is loaded before the fluxes.
+// while a row is worked on (the next row's without a condition: lanes and rows outside the grid
+// copy the nearest cell), and the update's other term is loaded before the fluxes.
 //
 // What bounds it: fixed-latency dependencies and the FP64 pipe (40 % of its cycles) at two
-// warps per scheduler.  4 x 1024^2 cells, harmonic: 886 -> 834 us a stage (4 x 256^2: 78 ->
-// 72); without the copies 884; three warps per scheduler (168 registers; both sides of a face
+// warps per scheduler.  4 x 1024^2 cells, harmonic: 886 -> 815 us a stage (4 x 256^2: 78 ->
+// 71); with copies under a condition and a state at rest in place of the missing cells 838,
+// without the copies 884; three warps per scheduler (168 registers; both sides of a face
 // one loop too, its states and partial sums in shared memory; no room for the copies, 20-100
 // bytes of spills) 930-1,020: the tighter allocation leaves less to issue between dependent
 // operations than the third warp brings.
@@ -74,11 +76,10 @@ __device__ __forceinline__ void exact_item(const StageArgs& a, const Work w, con
   const int rs = w.J0 >= 2 ? w.J0 - 2 : w.J0 - 1;
   int s0 = rs % 3;                 // window slot of row r
   auto u_fetch = [&](int rr) {
-    if (col_in && rr >= 0 && rr < nyp) {
-      const long long idx = (long long)rr * pitch + C + 1;
+    // lanes and rows outside the grid: the nearest cell's values, unused
+    const long long idx = (long long)min(rr, nyp - 1) * pitch + min(max(C, 0), nxp - 1) + 1;
 #pragma unroll
-      for (int n = 0; n < NV; n++) cp_async8(&win.Ua[n][lane], in + n * plane + idx);
-    }
+    for (int n = 0; n < NV; n++) cp_async8(&win.Ua[n][lane], in + n * plane + idx);
     cp_async_commit();
   };
   u_fetch(rs);
@@ -93,12 +94,8 @@ __device__ __forceinline__ void exact_item(const StageArgs& a, const Work w, con
       double U[NV], Q[NV];
       const bool ok = col_in && r >= 0 && r < nyp;
       cp_async_wait_all();
-      if (ok) {
 #pragma unroll
-        for (int n = 0; n < NV; n++) U[n] = win.Ua[n][lane];
-      } else {
-        benign(U);
-      }
+      for (int n = 0; n < NV; n++) U[n] = win.Ua[n][lane];
       if (HEUN == 1 && upd) {
 #pragma unroll
         for (int n = 0; n < NV; n++) cp_async8(&win.D0a[n][lane], d0src + n * plane + (long long)J * pitch + C + 1);
