@@ -235,7 +235,8 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
   // shared memory, without registers, while row J (= r-2) ... J+1 are worked on: loaded where
   // it is used, it was the longest wait of a row (the second longest in stage 2).  4 x 256^2 /
   // 512^2 / 1024^2 cells, harmonic: stage 1 34.9 / 99.9 / 333 -> 33.3 / 96.3 / 329 us, stage 2
-  // 34.8 / 98.5 / 320 -> 32.9 / 92.2 / 312 us; a step of 1024^2 666 -> 642 us.
+  // 34.8 / 98.5 / 320 -> 32.9 / 92.2 / 312 us; a step of 1024^2 666 -> 642 us (632 with a flux in
+  // every lane, below).
   constexpr bool PREFETCH = !TMA;
   // With bulk copies, the moments of row r+1 go to shared memory as well, and those of row J
   // are loaded again.  Where the window is not aligned for them, per-lane copies: one group per
@@ -396,7 +397,7 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
         hi[n] = fma(-0.5, S[n], p0);
         G[n] = fma(0.5, S[n], p0);            // lower state of the next face, parked in G
       }
-      if (face_now && ylane) {
+      if (face_now) {
         double lo[NV];
 #pragma unroll
         for (int n = 0; n < NV; n++) {
@@ -405,7 +406,7 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
         }
         const double lam = hll<2>(lo, hi, G);
         const int J = r - 2;
-        if (col_face && J >= 1 && J <= nyp - 3 && lam > lamy) lamy = lam;
+        if (ylane && col_face && J >= 1 && J <= nyp - 3 && lam > lamy) lamy = lam;
       } else {
 #pragma unroll
         for (int n = 0; n < NV; n++) win.lo[n][lane] = G[n];
@@ -440,12 +441,12 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
         lo[n] = fma(0.5, Sx[n], P0[n]);
         hi[n] = __shfl_down_sync(0xffffffffu, fma(-0.5, Sx[n], P0[n]), 1);
       }
-#pragma unroll
-      for (int n = 0; n < NV; n++) F[n] = 0.0;
-      if (lane >= 1 && lane <= 29) {
-        const double lam = hll<1>(lo, hi, F);
-        if (col_face && J >= 1 && J <= nyp - 3 && lam > lamx) lamx = lam;
-      }
+      // every lane forms a flux, those of lanes 0, 30 and 31 (and 0, 1, 30, 31 for y) unused: no
+      // branch and no state to give the others (512^2 cells, fast: a step 202 -> 196 us; in the
+      // bitwise march an unused lane's quotients would send the warp to the division's second
+      // path: 148 -> 171 us at 256^2)
+      const double lam = hll<1>(lo, hi, F);
+      if (lane >= 1 && lane <= 29 && col_face && J >= 1 && J <= nyp - 3 && lam > lamx) lamx = lam;
       double Fm[NV];
 #pragma unroll
       for (int n = 0; n < NV; n++) Fm[n] = __shfl_up_sync(0xffffffffu, F[n], 1);
@@ -494,7 +495,7 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
         }
       }
     }
-    if (face_now && ylane) {
+    if (face_now) {
 #pragma unroll
       for (int n = 0; n < NV; n++) win.G[n][lane] = G[n];
     }
