@@ -324,9 +324,9 @@ int mbm_ghost_map(const mbm_block_desc *blocks, int nblocks, int *entries, int c
  * Scratch: one file-scope device array of 320 KB (held by every GPU that loads
  * the library until the process exits): at most 64 blocks and 20,064 warp work
  * items (28-column strips x 32-row segments, e.g. 16 blocks of 1024^2); larger
- * inputs return MBM_EINVAL (smaller ones are cut into shorter segments or tiles).  Its device address is looked up by the first call on
- * each device, with that device current -- make that first call before any stream
- * capture.  Every call shares the array and clears what must start at zero; calls
+ * inputs return MBM_EINVAL (smaller ones are cut into shorter segments or tiles).
+ * Its device address is looked up by the first call on each device, with that
+ * device current -- make that first call before any stream capture.  Every call shares the array and clears what must start at zero; calls
  * that overlap on the GPU race.  Errors: mbm_last_error(NULL). */
 int mbm_stage_noalloc(const mbm_block_desc *blocks, int nblocks, const double *in,
                       const double *data0, double *out, double Kn, double F, int limiter,

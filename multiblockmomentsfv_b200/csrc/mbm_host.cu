@@ -807,8 +807,6 @@ extern "C" int mbm_create_batch(const mbm_block_desc* blocks, int nblocks, const
   return create_impl(glob, blk_case, cases, ncases, params, res, dir_off, ndir, nullptr, out);
 }
 
-// the context proper, from a block table whose ghost map is resolved; shard: the
-// exchange plan of a case split over ranks (nullptr otherwise)
 // whether a grid of this many tiles is advanced in tiles (MBM_TILES=1: any grid, 0: none)
 static bool tiles_pay(const mbm_ctx* c, long long tiles) {
   const char* env = getenv("MBM_TILES");
@@ -816,6 +814,8 @@ static bool tiles_pay(const mbm_ctx* c, long long tiles) {
   return tiles <= (c->fast ? TILE_MOST_FAST : c->lim == LIM_ANY ? TILE_MOST_EXACT_BATCH : TILE_MOST_EXACT);
 }
 
+// the context proper, from a block table whose ghost map is resolved; shard: the
+// exchange plan of a case split over ranks (nullptr otherwise)
 static int create_impl(const std::vector<mbm_block_desc>& glob, const std::vector<int>& blk_case,
                        const mbm_case_desc* cases, int ncases, const mbm_params* params,
                        const std::vector<Resolved>& res, const std::vector<int>& dir_off, int ndir,

@@ -25,11 +25,11 @@ constexpr int STRIP = 28;        // output columns per warp strip (32 lanes - 2 
 constexpr int TILE_ROWS = 4;     // output rows of a tile (28 x 4 cells, mbm_tile.cuh)
 // The most tiles of a grid that is advanced in tiles rather than by the row march: where the
 // two measured alike (a step of 4 x n^2 cells, harmonic, tiles / march in us):
-//   bitwise  n = 61: 23.6 / 51.3   192: 92 / 103   224 (2,052 tiles): 128 / 146   240: 144 / 145
-//   fast     n = 61: 14.6 / 33.3   192: 49 / 53    224: 68 / 68   256 (2,600 tiles): 97 / 78
+//   bitwise  n = 61: 23.0 / 49.7   192: 93 / 98    224 (2,052 tiles): 129 / 134   240 (2,196): 145 / 136
+//   fast     n = 61: 14.5 / 30.6   192 (1,372): 50.4 / 52.4   208 (1,696): 61.5 / 57.5   256: 86 / 74
 // A batch of several limiters costs the march more (its limiter is then taken at run time):
-//   bitwise  8 cases, 2,567 tiles: 159 / 172   4,668: 285 / 280;   fast  2,567: 88 / 83
-constexpr int TILE_MOST_EXACT = 2100, TILE_MOST_EXACT_BATCH = 4500, TILE_MOST_FAST = 1700;
+//   bitwise  8 cases, 2,567 tiles: 158 / 166   3,515: 213 / 216   4,169: 262 / 247;   fast  2,567: 87 / 81
+constexpr int TILE_MOST_EXACT = 2100, TILE_MOST_EXACT_BATCH = 3600, TILE_MOST_FAST = 1480;
 constexpr int CTA_WARPS = 4;     // warps per CTA of the persistent stage kernel
 constexpr int MAX_TRACE = 4096;  // progress records kept per case and Steps call
 
