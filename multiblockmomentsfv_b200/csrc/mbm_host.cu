@@ -240,7 +240,7 @@ static int wait_stream(mbm_ctx* c) {
 // where the stream's kernels and copies read them: the call needs no wait for the device
 // before the caller may have its buffer back.  Null: too large, or no room to be had.
 // 28 uploads of 40 KB: 559 -> 275 us; the set-up of a Steps call or a ghost fill: 26 -> 16 us.
-constexpr size_t RING_BYTES = 440 << 10, RING_MOST = 256 << 10, RING_RECORDS = 16 << 10;
+constexpr size_t RING_BYTES = 224 << 10, RING_MOST = 112 << 10, RING_RECORDS = 16 << 10;
 
 static void* ring_put(mbm_ctx* c, const void* src, size_t bytes) {
   if (bytes > RING_MOST || bytes > c->ring_bytes) return nullptr;
@@ -977,7 +977,7 @@ static int create_impl(const std::vector<mbm_block_desc>& glob, const std::vecto
   // controllers, maxima, queues, trace, per-block CFL
   CKC(cudaMalloc(&c->dcase, sizeof(CaseDev) * ncases));
   {
-    // all of the context's page-locked memory in one piece of less than 512 KB (unless the cases
+    // all of the context's page-locked memory in one piece of less than 256 KB (unless the cases
     // are many), the ring first: a context pays at most one page-locking of fresh memory, 0.8-2.6
     // ms whatever its size, and contexts that live side by side share it.  Without a block whose
     // state fits the ring, it takes case records only.
