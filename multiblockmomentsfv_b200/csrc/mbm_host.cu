@@ -579,8 +579,8 @@ static int push_cases(mbm_ctx* c) {
 // the per-segment warm-up (two extra primitive rows, one slope row, one face row)
 // against load balance over the persistent grid.  On first use of a problem shape
 // it times each Heun stage for each candidate on a uniform state at rest and keeps,
-// per stage, the fastest (the two stages have their own work tables: at 4 x 1024^2
-// stage 1 ran best at 24 rows, stage 2 at 29); the choice is cached per (strip rows,
+// per stage, the fastest (the two stages have their own work tables: at 4 x 1024^2,
+// fast, stage 1 runs best at 21-28 rows, stage 2 at 28-44); the choice is cached per (strip rows,
 // blocks, limiter mix, CTAs/SM) for the life of the process.  Lengths down to 2 rows: where
 // few warps are resident, a warp's march is the time, 4 rows of warm-up or not (a step of
 // 4 x 128^2 cells: 116 us bitwise and 54 us fast with 8 rows at the least, 75 and 43 with 2).
