@@ -403,8 +403,6 @@ static void build_work(mbm_ctx* c, double seg_rows, std::vector<Work>& w) {
   }
 }
 
-// rebuild the work table for segments of `seg` rows; the table lives in the same
-// device buffer (sized for 2-row segments)
 // work items of a segment length (host only; the count build_work makes)
 static long long count_items(const mbm_ctx* c, double seg_rows) {
   long long n = 0;
@@ -455,7 +453,8 @@ static int set_item_scatter(mbm_ctx* c, int k, const std::vector<Work>& work) {
   return MBM_OK;
 }
 
-// the work table of stage h (0, 1; -1: both) for segments of `seg` rows
+// the work table of stage h (0, 1; -1: both) for segments of `seg` rows, in the same device
+// buffer (sized for 2-row segments)
 static int set_segments(mbm_ctx* c, double seg, int h = -1) {
   for (int k = 0; k < 2; k++) {
     if (h >= 0 && k != h) continue;
