@@ -238,17 +238,24 @@ static int wait_stream(mbm_ctx* c) {
 
 // Small host inputs (a small block's state, a case record) are copied into the ring, from
 // where the stream's kernels and copies read them: the call needs no wait for the device
-// before the caller may have its buffer back.  Null: too large, or no room to be had.
+// before the caller may have its buffer back.  *p stays null where there is no room to be had.
 // 28 uploads of 40 KB: 559 -> 275 us; the set-up of a Steps call or a ghost fill: 26 -> 16 us.
+// A stream that is being captured is refused: the graph would read the ring when it is
+// launched, long after the bytes in it have changed.
 constexpr size_t RING_BYTES = 224 << 10, RING_MOST = 112 << 10, RING_RECORDS = 16 << 10;
 
-static void* ring_put(mbm_ctx* c, const void* src, size_t bytes) {
-  if (bytes > RING_MOST || bytes > c->ring_bytes) return nullptr;
-  if (c->ring_used + bytes > c->ring_bytes && wait_stream(c) != MBM_OK) return nullptr;   // empties it
-  void* p = c->ring + c->ring_used;
-  memcpy(p, src, bytes);
+static int ring_put(mbm_ctx* c, const void* src, size_t bytes, void** p) {
+  *p = nullptr;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  CK(cudaStreamIsCapturing(c->stream, &cs));
+  if (cs != cudaStreamCaptureStatusNone)
+    return fail(c, MBM_ECUDA, "the context's stream is being captured: host data cannot go into a graph");
+  if (bytes > RING_MOST || bytes > c->ring_bytes) return MBM_OK;
+  if (c->ring_used + bytes > c->ring_bytes && wait_stream(c) != MBM_OK) return MBM_OK;   // empties it
+  *p = c->ring + c->ring_used;
+  memcpy(*p, src, bytes);
   c->ring_used += (bytes + 255) & ~(size_t)255;
-  return p;
+  return MBM_OK;
 }
 
 static int kind_of(int code) { return code > 0 ? 0 : code == 0 ? 1 : code == -1 ? 2 : 3; }  // sync/open/wall/dirichlet
@@ -563,7 +570,10 @@ static cudaError_t launch_attempt(mbm_ctx* c, cudaGraphConditionalHandle h, int 
 }
 
 static int push_cases(mbm_ctx* c) {
-  if (const void* r = ring_put(c, c->hcase, sizeof(CaseDev) * c->ncase)) {
+  void* r;
+  const int st = ring_put(c, c->hcase, sizeof(CaseDev) * c->ncase, &r);
+  if (st) return st;
+  if (r) {
     CK(cudaMemcpyAsync(c->dcase, r, sizeof(CaseDev) * c->ncase, cudaMemcpyHostToDevice, c->stream));
     return MBM_OK;
   }
@@ -1203,7 +1213,10 @@ extern "C" int mbm_upload(mbm_ctx* c, int layer, int block, const double* cells)
   CK(cudaSetDevice(c->device));
   const BlockDev& d = c->hblk[block];
   const size_t bytes = sizeof(double) * d.nxp * d.nyp * NV;
-  if (const void* r = ring_put(c, cells, bytes)) {
+  void* r;
+  const int st = ring_put(c, cells, bytes, &r);
+  if (st) return st;
+  if (r) {
     CK(launch_aos_to_planes((const double*)r, c->buf[phys_of(c, layer, block)] + d.off, d.nxp, d.nyp, d.pitch, d.plane,
                             c->stream));
     return MBM_OK;
@@ -1229,7 +1242,9 @@ extern "C" int mbm_load_fields(mbm_ctx* c, int block, int single, const void* pa
   CK(cudaSetDevice(c->device));
   const BlockDev& d = c->hblk[block];
   const size_t bytes = (size_t)(d.nxp - 4) * (d.nyp - 4) * 10 * (single ? sizeof(float) : sizeof(double));
-  const void* r = ring_put(c, payload, bytes);
+  void* r;
+  const int st = ring_put(c, payload, bytes, &r);
+  if (st) return st;
   if (!r) CK(cudaMemcpyAsync(c->staging, payload, bytes, cudaMemcpyHostToDevice, c->stream));
   CK(launch_fields_to_planes(r ? r : c->staging, single, faithful, d.nxp, d.nyp, d.pitch, d.plane,
                              c->buf[phys_of(c, MBM_L_DATA, block)] + d.off, c->stream));
