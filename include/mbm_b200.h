@@ -109,7 +109,10 @@ int mbm_steps_batch_async(mbm_ctx *ctx, const double *t, const double *tend, dou
 int mbm_steps_batch_wait(mbm_ctx *ctx, double *t, int *nsteps, int *nrej);
 
 /* Copy one block of a layer between the host (array of structs, (nx+6)*(ny+6)*9
- * doubles, the reference's CVector layer, src/defs.h:42-44) and the device. */
+ * doubles, the reference's CVector layer, src/defs.h:42-44) and the device.  When
+ * mbm_upload returns the caller's buffer is free.  A small block (up to 112 KB here and in
+ * mbm_load_fields) is then queued on the context's stream, not yet on the device: an error
+ * of the device is reported by the next call that waits. */
 int mbm_upload(mbm_ctx *ctx, int layer, int block, const double *cells);
 int mbm_download(mbm_ctx *ctx, int layer, int block, double *cells);
 

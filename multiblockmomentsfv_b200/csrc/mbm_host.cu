@@ -238,7 +238,7 @@ static int wait_stream(mbm_ctx* c) {
 
 // Small host inputs (a small block's state, a case record) are copied into the ring, from
 // where the stream's kernels and copies read them: the call needs no wait for the device
-// before the caller may have its buffer back.  *p stays null where there is no room to be had.
+// before the caller may have its buffer back.  *p stays null where they are too large for it.
 // 28 uploads of 40 KB: 559 -> 275 us; the set-up of a Steps call or a ghost fill: 26 -> 16 us.
 // A stream that is being captured is refused: the graph would read the ring when it is
 // launched, long after the bytes in it have changed.
@@ -251,7 +251,10 @@ static int ring_put(mbm_ctx* c, const void* src, size_t bytes, void** p) {
   if (cs != cudaStreamCaptureStatusNone)
     return fail(c, MBM_ECUDA, "the context's stream is being captured: host data cannot go into a graph");
   if (bytes > RING_MOST || bytes > c->ring_bytes) return MBM_OK;
-  if (c->ring_used + bytes > c->ring_bytes && wait_stream(c) != MBM_OK) return MBM_OK;   // empties it
+  if (c->ring_used + bytes > c->ring_bytes) {
+    const int st = wait_stream(c);           // empties it
+    if (st) return st;
+  }
   *p = c->ring + c->ring_used;
   memcpy(*p, src, bytes);
   c->ring_used += (bytes + 255) & ~(size_t)255;
@@ -580,8 +583,7 @@ static int push_cases(mbm_ctx* c) {
   CK(cudaMemcpyAsync(c->dcase, c->hcase, sizeof(CaseDev) * c->ncase, cudaMemcpyHostToDevice, c->stream));
   // the records are pinned: the copy reads them when the stream reaches it, so the
   // host must not change them before then
-  CK(cudaStreamSynchronize(c->stream));
-  return MBM_OK;
+  return wait_stream(c);
 }
 
 // Autotuner: the stage kernel's work-item length (rows per warp segment) trades

@@ -45,3 +45,29 @@ def test_payload_buffer_reuse(dtype):
             p[...] = 0
         for b in range(4):
             H.assert_bitwise(s.download(0, b), want[b], f"block {b}")
+
+
+@pytest.mark.parametrize("ncase", [1, 600])
+def test_a_wait_for_room_that_runs_out_is_reported(monkeypatch, ncase):
+    """The ring is full and the stream busy for longer than MBM_WAIT_TIMEOUT_S: the call that
+    needs room returns MBM_ETIMEOUT, as it does where the records of many cases do not fit the
+    ring, and the context works again once the stream has caught up."""
+    import torch
+    from multiblockmomentsfv_b200 import _abi, scenario as sc
+    st = torch.cuda.Stream()
+    d = bf.Deck(Kn=0.02, limiter=4)
+    d.blocks = [bf.Block(1, 0.0, 1.0, 0.0, 1.0, 8, 8, (0, 0, 0, 0))]
+    cases = [(d, sc.Scenario.seeded_quadrant(k)) for k in range(ncase)]
+    with sv.BatchSolver(cases, stream=st.cuda_stream) as s:
+        s.initialise()
+        monkeypatch.setenv("MBM_WAIT_TIMEOUT_S", "0.02")
+        with torch.cuda.stream(st):
+            torch.cuda._sleep(1_500_000_000)                # about 0.8 s
+        with pytest.raises(_abi.MBMError) as e:
+            for _ in range(4000):
+                _abi.check(s.L.mbm_set_physics(s.ctx, 0.02, 0.0), s.ctx)
+        assert e.value.status == _abi.MBM_ETIMEOUT
+        monkeypatch.setenv("MBM_WAIT_TIMEOUT_S", "60")
+        _abi.check(s.L.mbm_set_physics(s.ctx, 0.02, 0.0), s.ctx)
+        t, n, _ = s.steps(0.0, 1.0, max_steps=2)
+        assert np.all(n == 2)
