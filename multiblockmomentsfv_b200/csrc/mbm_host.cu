@@ -124,6 +124,7 @@ struct mbm_ctx {
   int tile_grid = 0;
   unsigned* dsync = nullptr;        // tile_steps: TileLoop::sync (4 words) and ::lam behind it
   unsigned* hsync = nullptr;        // pinned: whether one of its waits ran out
+  int tile_drop = 0;                // failure-detection test: the next loop's CTA 0 never arrives
   Work* dwork = nullptr;            // the work tables of the two Heun stages, max_items apart
   long long max_items = 0;
   int nwork[2] = {0, 0};
@@ -1042,6 +1043,10 @@ static int create_impl(const std::vector<mbm_block_desc>& glob, const std::vecto
     c->tile_grid = (int)std::min<long long>(tiles, (long long)c->nsm * tile_ctas);
     c->tile_loop = !c->adjoint && !shard && tiles <= (long long)TILE_MAX * c->tile_grid;
     CKC(cudaMalloc(&c->dsync, tile_scratch(c)));
+    // failure-detection test hook: one CTA of the first step loop leaves without arriving at
+    // the grid barrier, so that the others' bounded waits (20 ms then) run out
+    const char* drop = getenv("MBM_TILE_TEST_DROP");
+    c->tile_drop = drop && atoi(drop) == 1;
   }
   c->max_items = std::max<long long>(1, max_items);
   CKC(cudaMalloc(&c->dwork, sizeof(Work) * 2 * c->max_items));
@@ -1395,6 +1400,7 @@ extern "C" int mbm_steps_batch_async(mbm_ctx* c, const double* t, const double* 
   if (c->sharded) return fail(c, MBM_EINVAL, "mbm_steps: the context holds part of a sharded case (mbm_shard_*)");
   CK(cudaSetDevice(c->device));
   bool any = false;
+  *c->hsync = 0;
   for (int k = 0; k < c->ncase; k++) {
     CaseDev& h = c->hcase[k];
     h.t = t[k];
@@ -1429,6 +1435,9 @@ extern "C" int mbm_steps_batch_async(mbm_ctx* c, const double* t, const double* 
     L.trace = c->dtrace;
     L.sync = c->dsync;
     L.lam = (unsigned long long*)(c->dsync + 4);
+    L.drop = c->tile_drop;
+    L.wait_ns = c->tile_drop ? 20000000ull : TILE_WAIT_NS;
+    c->tile_drop = 0;
     CK(cudaMemsetAsync(c->dsync, 0, tile_scratch(c), c->stream));
     CK(c->fast ? fastmath::launch_tile_steps(L, c->tile_grid, c->stream)
                : bitwise::launch_tile_steps(L, c->tile_grid, c->stream));
@@ -1459,7 +1468,11 @@ extern "C" int mbm_steps_batch_wait(mbm_ctx* c, double* t, int* nsteps, int* nre
   int st;
   CK(cudaMemcpyAsync(c->hcase, c->dcase, sizeof(CaseDev) * c->ncase, cudaMemcpyDeviceToHost, c->stream));
   if ((st = wait_stream(c))) return st;
-  if (c->hsync && *c->hsync) return fail(c, MBM_ETIMEOUT, "a bounded wait of the step loop's grid barrier ran out");
+  if (*c->hsync) {      // the records on the device are those the loop started from
+    for (int k = 0; k < c->ncase; k++)
+      if (!c->hcase[k].done) c->hcase[k].status = 3;
+    return fail(c, MBM_ETIMEOUT, "a bounded wait of the step loop's grid barrier ran out");
+  }
   int worst = 0;
   for (int k = 0; k < c->ncase; k++) {
     const CaseDev& h = c->hcase[k];

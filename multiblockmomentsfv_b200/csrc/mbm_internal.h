@@ -138,7 +138,10 @@ struct TileLoop {      // the step loop of tile_steps (mbm_tile.cuh)
   double* trace;
   unsigned long long* lam;   // three sets of the blocks' maxima
   unsigned* sync;            // [0] arrivals at the grid barrier, [2] a wait ran out, [3] cases done
+  unsigned long long wait_ns;   // a wait at the grid barrier gives up after this much device time
+  int drop;                  // failure-detection test only: CTA 0 leaves without arriving
 };
+constexpr unsigned long long TILE_WAIT_NS = 10000000000ull;
 
 constexpr int TMAP_BYTES = 128;   // sizeof(CUtensorMap)
 

@@ -384,9 +384,8 @@ cudaError_t launch_tiles(const StageArgs& a, cudaStream_t s) {
 
 // ------------------------------------------------------------------- the step loop --
 // Barrier over the grid, `phase` the number of barriers passed with this one.  A wait gives up
-// after TILE_WAIT_NS of device time (sync[2] is then set and the CTA returns).  Thread 0's
+// after wait_ns of device time (sync[2] is then set and the CTA returns).  Thread 0's
 // release and acquire order the CTA's accesses, as in a cooperative grid's own barrier.
-constexpr unsigned long long TILE_WAIT_NS = 10000000000ull;
 
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
   unsigned v;
@@ -394,7 +393,7 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
   return v;
 }
 
-__device__ __forceinline__ bool tile_barrier(unsigned* sync, unsigned phase) {
+__device__ __forceinline__ bool tile_barrier(unsigned* sync, unsigned phase, unsigned long long wait_ns) {
   __syncthreads();
   int ok = 1;
   if (threadIdx.x == 0) {
@@ -405,7 +404,7 @@ __device__ __forceinline__ bool tile_barrier(unsigned* sync, unsigned phase) {
       if ((k & 1023u) != 1023u) continue;
       const unsigned long long t = global_ns();
       if (t0 == 0) t0 = t;
-      if (t - t0 > TILE_WAIT_NS || k > (1u << 30)) { ok = 0; break; }
+      if (t - t0 > wait_ns || k > (1u << 30)) { ok = 0; break; }
     }
     if (!ok) atomicExch(sync + 2, 1u);
   }
@@ -436,6 +435,7 @@ __global__ void __launch_bounds__(TILE_THREADS, TILE_CTAS) tile_steps(const Tile
   TileShared& sh = *reinterpret_cast<TileShared*>(stage_shared);
   TileLoopShared& ls = *reinterpret_cast<TileLoopShared*>(stage_shared + sizeof(TileShared));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (L.drop && blockIdx.x == 0) return;
   StageArgs a = L.st;
   if (tid < TILE_MAX) {
     const int w = blockIdx.x + tid * gridDim.x;
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(TILE_THREADS, TILE_CTAS) tile_steps(const Tile
       if (!c.done)
         tile_stage<0>(a, m.w, m.B, m.goff, TileCase{c.dt, c.F, c.Kn, c.limiter, c.cur, c.nstep > 0}, sh);
     }
-    if (!tile_barrier(L.sync, ++phase)) return;
+    if (!tile_barrier(L.sync, ++phase, L.wait_ns)) return;
     if (L.ncase > 1) {      // every case done, as of the last attempt
       if (tid == 0) ls.stop = __ldcg(L.sync + 3) == (unsigned)L.ncase;
       __syncthreads();
@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(TILE_THREADS, TILE_CTAS) tile_steps(const Tile
       const CaseDev& c = ls.ctl[m.slot];
       if (!c.done) tile_stage<1>(a, m.w, m.B, m.goff, TileCase{c.dt, c.F, c.Kn, c.limiter, c.cur, true}, sh);
     }
-    if (!tile_barrier(L.sync, ++phase)) return;
+    if (!tile_barrier(L.sync, ++phase, L.wait_ns)) return;
     // controllers: a warp per case of this CTA
     for (int j = warp; j < ls.ncase; j += TILE_THREADS / 32) {
       CaseDev& c = ls.ctl[j];
@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(TILE_THREADS, TILE_CTAS) tile_steps(const Tile
   // the owners' records, then SetBoundary of the layers the loop wrote: TMP, DATA if a step was
   // accepted, and the third layer unless it still is the state the call started from
   if (tid < ls.ncase && ls.owner[tid]) a.cases[ls.id[tid]] = ls.ctl[tid];
-  if (!tile_barrier(L.sync, ++phase)) return;
+  if (!tile_barrier(L.sync, ++phase, L.wait_ns)) return;
   for (int i = blockIdx.x * blockDim.x + tid; i < 3 * L.nghost; i += gridDim.x * blockDim.x) {
     const int which = i / L.nghost;
     const GhostEntry e = a.ghosts[i - which * L.nghost];

@@ -312,7 +312,8 @@ class BatchSolver:
         return tt, np.array(ns[:]), np.array(nr[:])
 
     def case_status(self) -> np.ndarray:
-        """Per-case status of the last steps() call (MBM_OK, MBM_ENONFINITE, MBM_ESTEPLIMIT)."""
+        """Per-case status of the last steps() call (MBM_OK, MBM_ENONFINITE, MBM_ESTEPLIMIT,
+        MBM_ETIMEOUT)."""
         n = len(self.cases)
         s = (C.c_int * n)()
         _abi.check(self.L.mbm_case_status(self.ctx, s, n), self.ctx)
