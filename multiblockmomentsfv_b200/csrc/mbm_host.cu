@@ -46,7 +46,7 @@ cudaError_t launch_shard_cfl(const CaseDev* cases, const BlockDev* blk, int nblk
                              double* out, cudaStream_t s);
 cudaError_t launch_control_ext(CaseDev* cases, const BlockDev* blk, unsigned long long* lam, double* trace,
                                int* queues, const double* cfl_ext, cudaStream_t s);
-cudaError_t launch_control(CaseDev* cases, int ncases, const BlockDev* blk, unsigned long long* lam,
+cudaError_t launch_control(CaseDev* cases, int ncases, const BlockDev* blk, int nblk, unsigned long long* lam,
                            double* trace, int* queues, cudaGraphConditionalHandle h, int use_handle,
                            cudaStream_t s);
 cudaError_t launch_frozen_prep(CaseDev* cases, const double* ddt, int* queues, cudaStream_t s);
@@ -567,7 +567,8 @@ static cudaError_t launch_attempt(mbm_ctx* c, cudaGraphConditionalHandle h, int 
   if (g && (e = launch_ghost(c->dblk, c->dcase, c->dghost, c->nghost, c->buf, c->ddir, SEL_TMP, c->stream))) return e;
   if ((e = launch_stages(c, 1, SEL_TMP, SEL_CUR, SEL_OTHER, 1, nullptr, true))) return e;
   if (g && (e = launch_ghost(c->dblk, c->dcase, c->dghost, c->nghost, c->buf, c->ddir, SEL_OTHER, c->stream))) return e;
-  if ((e = launch_control(c->dcase, c->ncase, c->dblk, c->dlam, c->dtrace, c->dqueue, h, use_handle, c->stream)))
+  if ((e = launch_control(c->dcase, c->ncase, c->dblk, c->nblk, c->dlam, c->dtrace, c->dqueue, h, use_handle,
+                          c->stream)))
     return e;
   if (c->adjoint) return launch_ckpt(c->dcase, c->buf[0], c->buf[1], c->buf[2], c->layer_elems, 4 * c->nsm, c->stream);
   return cudaSuccess;

@@ -33,10 +33,10 @@ __global__ void ghost_kernel(const BlockDev* __restrict__ blk, const CaseDev* __
 // one Steps iteration's bookkeeping (control_cases, mbm_step.cuh)
 __global__ void control_kernel(CaseDev* cases, int ncases, const BlockDev* __restrict__ blk,
                                unsigned long long* lam, double* trace, int* queues,
-                               cudaGraphConditionalHandle h, int use_handle, const double* cfl_ext) {
+                               cudaGraphConditionalHandle h, int use_handle, const double* cfl_ext, int width) {
   pdl_enter();
   if (threadIdx.x < 10) queues[threadIdx.x] = 0;  // work counters [stage][limiter]
-  const int live = control_cases(cases, ncases, blk, lam, trace, cfl_ext);
+  const int live = control_cases(cases, ncases, blk, lam, trace, cfl_ext, width);
   if (use_handle && threadIdx.x == 0) cudaGraphSetConditional(h, live ? 1u : 0u);
 }
 
@@ -286,7 +286,7 @@ cudaError_t launch_shard_cfl(const CaseDev* cases, const BlockDev* blk, int nblk
 
 cudaError_t launch_control_ext(CaseDev* cases, const BlockDev* blk, unsigned long long* lam, double* trace,
                                int* queues, const double* cfl_ext, cudaStream_t s) {
-  control_kernel<<<1, 256, 0, s>>>(cases, 1, blk, lam, trace, queues, cudaGraphConditionalHandle{}, 0, cfl_ext);
+  control_kernel<<<1, 256, 0, s>>>(cases, 1, blk, lam, trace, queues, cudaGraphConditionalHandle{}, 0, cfl_ext, 32);
   return cudaGetLastError();
 }
 
@@ -299,11 +299,11 @@ cudaError_t launch_ghost(const BlockDev* blk, const CaseDev* cases, const GhostE
                   buf[1], buf[2], dirichlet, recv, sel);
 }
 
-cudaError_t launch_control(CaseDev* cases, int ncases, const BlockDev* blk, unsigned long long* lam,
+cudaError_t launch_control(CaseDev* cases, int ncases, const BlockDev* blk, int nblk, unsigned long long* lam,
                            double* trace, int* queues, cudaGraphConditionalHandle h, int use_handle,
                            cudaStream_t s) {
   return launch_k(control_kernel, dim3(1), dim3(256), 0, s, cases, ncases, blk, lam, trace, queues, h, use_handle,
-                  (const double*)nullptr);
+                  (const double*)nullptr, control_width(ncases, nblk));
 }
 
 cudaError_t launch_stage_cfl(const BlockDev* blk, int nblk, const CaseDev* cases,

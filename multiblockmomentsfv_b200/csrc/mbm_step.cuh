@@ -38,17 +38,19 @@ __device__ __forceinline__ void ghost_fill(const BlockDev* __restrict__ blk, con
 }
 
 // CFL of an attempt of case c (src/Main.c:253-283): the maximum over stages and blocks of
-// dt*lx/dx + dt*ly/dy + prod, a warp's lanes over the blocks (the maximum is order-free).
+// dt*lx/dx + dt*ly/dy + prod, `width` lanes (those of mask) over the blocks (the maximum is
+// order-free).
 // The values are >= 0 or NaN, which never passes a '>' test.  bad: a maximum that tile_steps
 // flagged (a NaN or infinity was written).
 constexpr unsigned long long LAM_NONFINITE = ~0ull;
 
 __device__ __forceinline__ double case_cfl(const CaseDev& c, const BlockDev* __restrict__ blk,
-                                           const unsigned long long* lam, int lane, bool& bad) {
+                                           const unsigned long long* lam, int lane, bool& bad, int width = 32,
+                                           unsigned mask = 0xffffffffu) {
   const double dt = c.dt;
   bad = false;
   double cfl = 0.0;
-  for (int b = c.blk0 + lane; b < c.blk0 + c.nblk; b += 32) {
+  for (int b = c.blk0 + lane; b < c.blk0 + c.nblk; b += width) {
     const unsigned long long* s = lam + (size_t)b * 6;
     double v[6];
 #pragma unroll
@@ -63,9 +65,9 @@ __device__ __forceinline__ double case_cfl(const CaseDev& c, const BlockDev* __r
     if (v1 > cfl) cfl = v1;
     if (v2 > cfl) cfl = v2;
   }
-  const unsigned h = (unsigned)__double2hiint(cfl), hm = __reduce_max_sync(0xffffffffu, h);
-  const unsigned lm = __reduce_max_sync(0xffffffffu, h == hm ? (unsigned)__double2loint(cfl) : 0u);
-  bad = __any_sync(0xffffffffu, bad);
+  const unsigned h = (unsigned)__double2hiint(cfl), hm = __reduce_max_sync(mask, h);
+  const unsigned lm = __reduce_max_sync(mask, h == hm ? (unsigned)__double2loint(cfl) : 0u);
+  bad = __any_sync(mask, bad);
   return __hiloint2double((int)hm, (int)lm);
 }
 
@@ -113,19 +115,31 @@ __device__ __forceinline__ void control_case(CaseDev& cs, double cfl, double* tr
   }
 }
 
-// The controllers of every case, called by all threads of one CTA, a warp per case; clears
-// the maxima.  Returns, in every thread, whether a case is still live.
+// the lanes of a case's controller: the cases' mean number of blocks, up to a power of two, at most 32
+inline int control_width(int ncases, int nblk) {
+  int w = 1;
+  while (w < 32 && (long long)w * ncases < nblk) w *= 2;
+  return w;
+}
+
+// The controllers of every case, called by all threads of one CTA; clears the maxima.  Returns,
+// in every thread, whether a case is still live.  A case gets `width` lanes (control_width): one
+// case of 28 blocks a warp, a batch of one-block cases a thread each.  A chain of dependent loads and divisions per case, 2.4 us, is
+// what bounds it, so many cases must run side by side: a step attempt of 512 one-block cases of
+// 24^2 cells, fast, 279 us with a warp per case, 124 like this.
 __device__ __forceinline__ int control_cases(CaseDev* cases, int ncases, const BlockDev* __restrict__ blk,
-                                             unsigned long long* lam, double* trace, const double* cfl_ext) {
+                                             unsigned long long* lam, double* trace, const double* cfl_ext,
+                                             int width) {
   int live = 0;
-  const int lane = threadIdx.x & 31;
-  for (int c = threadIdx.x >> 5; c < ncases; c += blockDim.x >> 5) {
+  const int lane = threadIdx.x & (width - 1);
+  const unsigned mask = (width == 32 ? 0xffffffffu : (1u << width) - 1u) << (threadIdx.x & 31 & ~(width - 1));
+  for (int c = threadIdx.x / width; c < ncases; c += blockDim.x / width) {
     CaseDev& cs = cases[c];
     if (cs.done) continue;
     bool flagged;      // (never here: the stages' kernels flag cs.nonfinite)
-    const double cfl = case_cfl(cs, blk, lam, lane, flagged);
-    for (int q = lane; q < 6 * cs.nblk; q += 32) lam[(size_t)cs.blk0 * 6 + q] = 0ull;
-    __syncwarp();
+    const double cfl = case_cfl(cs, blk, lam, lane, flagged, width, mask);
+    for (int q = lane; q < 6 * cs.nblk; q += width) lam[(size_t)cs.blk0 * 6 + q] = 0ull;
+    __syncwarp(mask);
     if (lane != 0) continue;
     // a case split over ranks brings the max over all ranks (single-case contexts)
     control_case(cs, cfl_ext ? *cfl_ext : cfl, trace + (size_t)c * MAX_TRACE * 4);
