@@ -300,6 +300,12 @@ int mbm_dependent_launch(mbm_ctx *ctx, int *on);
  * src < 0 is Dirichlet row -(src+1), flags bit 0/1 = x/y wall sign.  Needs no GPU. */
 int mbm_ghost_map(const mbm_block_desc *blocks, int nblocks, int *entries, int cap, int *n);
 
+/* Host-only: the segment lengths (rows) that context creation would time for a block table,
+ * given the resident warps of the two stages on the device; *n is their number.  No counterpart
+ * in the reference.  Needs no GPU. */
+int mbm_tune_lengths(const mbm_block_desc *blocks, int nblocks, int warps1, int warps2, double *lengths,
+                     int cap, int *n);
+
 /* One Heun stage -- Update (src/Main.c:297-396) of every block -- on device buffers
  * the caller owns, allocating no device memory: no cudaMalloc, cudaFree or
  * allocating library routine is called.  No counterpart in the reference (its

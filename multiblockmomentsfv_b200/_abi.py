@@ -23,7 +23,7 @@ EXPORTS = (
     "mbm_time_stage", "mbm_trace", "mbm_attempts", "mbm_case_status", "mbm_config",
     "mbm_create_batch", "mbm_steps_batch", "mbm_trace_case", "mbm_stage_noalloc", "mbm_bulk_copies", "mbm_load_fields", "mbm_config_stage", "mbm_ghost_scatter", "mbm_dependent_launch", "mbm_set_functional",
     "mbm_adjoint_run", "mbm_replay", "mbm_set_physics", "mbm_output_fields",
-    "mbm_ghost_map", "mbm_strerror", "mbm_last_error", "mbm_version",
+    "mbm_ghost_map", "mbm_tune_lengths", "mbm_strerror", "mbm_last_error", "mbm_version",
     "mbm_shard_plan", "mbm_create_sharded", "mbm_shard_buffers", "mbm_shard_set_dirichlet",
     "mbm_shard_begin", "mbm_shard_stage",
     "mbm_shard_pack", "mbm_shard_fill", "mbm_shard_cfl", "mbm_shard_control", "mbm_shard_end",
@@ -122,6 +122,7 @@ def lib(path: str = None):
     L.mbm_stage_noalloc.argtypes = [P(BlockDesc), C.c_int, vp, vp, vp, C.c_double, C.c_double, C.c_int,
                                     C.c_double, C.c_int, dp, vp]
     L.mbm_ghost_map.argtypes = [P(BlockDesc), C.c_int, P(C.c_int), C.c_int, P(C.c_int)]
+    L.mbm_tune_lengths.argtypes = [P(BlockDesc), C.c_int, C.c_int, C.c_int, dp, C.c_int, P(C.c_int)]
     L.mbm_strerror.restype = C.c_char_p
     L.mbm_strerror.argtypes = [C.c_int]
     L.mbm_last_error.restype = C.c_char_p

@@ -415,10 +415,10 @@ static void build_work(mbm_ctx* c, double seg_rows, std::vector<Work>& w) {
 }
 
 // work items of a segment length (host only; the count build_work makes)
-static long long count_items(const mbm_ctx* c, double seg_rows) {
+static long long count_items(const std::vector<BlockDev>& blk, double seg_rows) {
   long long n = 0;
-  for (int b = 0; b < c->nblk; b++) {
-    const int nfx = c->hblk[b].nxp - 3, nfy = c->hblk[b].nyp - 3;
+  for (const BlockDev& d : blk) {
+    const int nfx = d.nxp - 3, nfy = d.nyp - 3;
     n += (long long)((nfx + STRIP - 1) / STRIP) * std::max(1, (int)std::ceil(nfy / seg_rows - 1e-9));
   }
   return n;
@@ -620,12 +620,46 @@ static int time_each_stage(mbm_ctx* c, cudaEvent_t e0, cudaEvent_t e1, float* ms
   return MBM_OK;
 }
 
-static int autotune(mbm_ctx* c) {
-  long long strip_rows = 0, cells = 0;
-  for (auto& d : c->hblk) {
-    strip_rows += (long long)((d.nxp - 3 + STRIP - 1) / STRIP) * (d.nyp - 3);
-    cells += (long long)d.nxp * d.nyp;
+// The lengths the tuner times, for W1 and W2 resident warps of the two stages.  Short segments
+// buy parallelism on small grids, long ones save warm-up rows.  The persistent grid's warps
+// take the items from a queue, so the time jumps with the item count: besides every even
+// length, each wave count k gets the shortest length whose items fill k waves of the resident
+// warps without a partial one (the segment count is ceil(rows / length), so these lengths are
+// fractional).  4 x 1024^2 cells: 22 rows (6,956 items, 3.92 waves) 3 % faster than 24, 20 rows
+// 5 % slower, 21.4 rows (7,104 items, 4 waves) 1.7 % faster than 22.
+// Lengths below 8 rows, 4 rows of warm-up each, won up to 1.1 waves of 8-row items on equal
+// blocks (4 x 256^2 cells fast: 6 rows) and, at 6 and 7 rows, up to 4.7 waves on ragged ones (28
+// blocks of 240 x 80 cells and the 12-case batch, bitwise): all of them below 2 waves, 6 and 7
+// rows below 5.  Timing all of them everywhere made the first creation at 4 x 1024^2 cells
+// 226 ms fast and 656 bitwise, 125 and 261 like this (512^2: 50 and 105, now 37 and 72), for
+// lengths that never won.
+static std::vector<double> tune_lengths(const std::vector<BlockDev>& blk, long long W1, long long W2) {
+  std::vector<double> cand;
+  const long long n8 = count_items(blk, 8.0), W0 = std::min(W1, W2);
+  const bool small = n8 < 2 * W0;
+  for (int seg = small ? 2 : n8 < 5 * W0 ? 6 : 8; seg < 8; seg++) cand.push_back(seg);
+  for (int seg = 8; seg <= 64; seg += 2) cand.push_back(seg);
+  for (int h = 0; h < 2; h++) {
+    if (h == 1 && W1 == W2) break;
+    const long long W = h ? W2 : W1;
+    const double shortest = small ? 2.0 : 8.0;
+    const long long most = count_items(blk, shortest), least = count_items(blk, 64.0);
+    for (long long k = (least + W - 1) / W; k * W < most && k <= 64; k++) {
+      double lo = shortest, hi = 64.0;         // count_items(hi) <= k W < count_items(lo)
+      for (int it = 0; it < 40; it++) {
+        const double mid = 0.5 * (lo + hi);
+        if (count_items(blk, mid) <= k * W) hi = mid;
+        else lo = mid;
+      }
+      cand.push_back(hi);
+    }
   }
+  return cand;
+}
+
+static int autotune(mbm_ctx* c) {
+  long long strip_rows = 0;
+  for (auto& d : c->hblk) strip_rows += (long long)((d.nxp - 3 + STRIP - 1) / STRIP) * (d.nyp - 3);
   const auto key = std::make_tuple(strip_rows, c->nblk, c->lim,
                                    ((c->ctas_per_sm[0] * 256 + c->ctas_per_sm[1]) * c->cta_warps) * 2 + c->fast);
   {
@@ -651,30 +685,8 @@ static int autotune(mbm_ctx* c) {
   CK(cudaEventCreate(&ev.e[1]));
   double best[2] = {32, 32};
   float best_ms[2] = {1e30f, 1e30f};
-  // short segments buy parallelism on small grids, long ones save warm-up rows.  The
-  // persistent grid's warps take the items from a queue, so the time jumps with the item
-  // count: besides every even length, each wave count k gets the shortest length whose
-  // items fill k waves of the resident warps without a partial one (the segment count is
-  // ceil(rows / length), so these lengths are fractional).  4 x 1024^2 cells: 22 rows
-  // (6,956 items, 3.92 waves) 3 % faster than 24, 20 rows 5 % slower, 21.4 rows (7,104
-  // items, 4 waves) 1.7 % faster than 22.
-  std::vector<double> cand;
-  for (int seg = 2; seg < 8; seg++) cand.push_back(seg);
-  for (int seg = 8; seg <= 64; seg += 2) cand.push_back(seg);
-  for (int h = 0; h < 2; h++) {              // the resident warps of each stage
-    if (h == 1 && c->ctas_per_sm[1] == c->ctas_per_sm[0]) break;
-    const long long W = (long long)c->nsm * c->ctas_per_sm[h] * c->cta_warps;
-    const long long most = count_items(c, 2.0), least = count_items(c, 64.0);
-    for (long long k = (least + W - 1) / W; k * W < most && k <= 64; k++) {
-      double lo = 2.0, hi = 64.0;              // count_items(hi) <= k W < count_items(lo)
-      for (int it = 0; it < 40; it++) {
-        const double mid = 0.5 * (lo + hi);
-        if (count_items(c, mid) <= k * W) hi = mid;
-        else lo = mid;
-      }
-      cand.push_back(hi);
-    }
-  }
+  const std::vector<double> cand = tune_lengths(
+      c->hblk, (long long)c->nsm * c->ctas_per_sm[0] * c->cta_warps, (long long)c->nsm * c->ctas_per_sm[1] * c->cta_warps);
   for (double seg : cand) {             // each stage keeps its own fastest length
     st = set_segments(c, seg);
     float ms[2] = {0.f, 0.f};
@@ -2238,6 +2250,22 @@ extern "C" int mbm_ghost_map(const mbm_block_desc* blocks, int nblocks, int* ent
       entries[4 * i + 3] = res[i].src_blk | (res[i].flags << 16);
     }
   }
+  return MBM_OK;
+}
+
+extern "C" int mbm_tune_lengths(const mbm_block_desc* blocks, int nblocks, int warps1, int warps2, double* lengths,
+                                int cap, int* n) {
+  std::string why;
+  if (validate(blocks, nblocks, why) != MBM_OK) return fail(nullptr, MBM_EINVAL, why);
+  if (warps1 < 1 || warps2 < 1) return fail(nullptr, MBM_EINVAL, "mbm_tune_lengths: bad warp count");
+  std::vector<BlockDev> blk(nblocks);
+  for (int b = 0; b < nblocks; b++) {
+    blk[b].nxp = blocks[b].nx + 2 * NG;
+    blk[b].nyp = blocks[b].ny + 2 * NG;
+  }
+  const std::vector<double> cand = tune_lengths(blk, warps1, warps2);
+  if (n) *n = (int)cand.size();
+  for (int i = 0; lengths && i < cap && i < (int)cand.size(); i++) lengths[i] = cand[i];
   return MBM_OK;
 }
 
