@@ -840,6 +840,44 @@ static bool tiles_pay(const mbm_ctx* c, long long tiles) {
   return tiles <= (c->fast ? TILE_MOST_FAST : c->lim == LIM_ANY ? TILE_MOST_EXACT_BATCH : TILE_MOST_EXACT);
 }
 
+// the step loop as a graph: while (any case live) { stage 1; fill TMP; stage 2; fill NEW; control }
+// (in tiles without checkpoints: tile_steps, and this one only where the device refuses that)
+static cudaError_t step_graph(mbm_ctx* c) {
+  auto build_graph = [&]() -> cudaError_t {
+    if (c->gexec) cudaGraphExecDestroy(c->gexec);
+    if (c->graph) cudaGraphDestroy(c->graph);
+    c->gexec = nullptr;
+    c->graph = nullptr;
+    cudaError_t e;
+    cudaGraphConditionalHandle h;
+    if ((e = cudaGraphCreate(&c->graph, 0))) return e;
+    if ((e = cudaGraphConditionalHandleCreate(&h, c->graph, 1, cudaGraphCondAssignDefault))) return e;
+    cudaGraphNodeParams np = {};
+    np.type = cudaGraphNodeTypeConditional;
+    np.conditional.handle = h;
+    np.conditional.type = cudaGraphCondTypeWhile;
+    np.conditional.size = 1;
+    cudaGraphNode_t node;
+    if ((e = cudaGraphAddNode(&node, c->graph, nullptr, 0, &np))) return e;
+    cudaGraph_t body = np.conditional.phGraph_out[0];
+    if ((e = cudaStreamBeginCaptureToGraph(c->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)))
+      return e;
+    const cudaError_t e1 = launch_attempt(c, h, 1);
+    cudaGraph_t captured = nullptr;
+    const cudaError_t e2 = cudaStreamEndCapture(c->stream, &captured);
+    if (e1) return e1;
+    if (e2) return e2;
+    return cudaGraphInstantiate(&c->gexec, c->graph, 0);
+  };
+  cudaError_t eg = build_graph();
+  if (eg != cudaSuccess && c->pdl) {   // without programmatic launches, once more
+    cudaGetLastError();
+    c->pdl = false;
+    eg = build_graph();
+  }
+  return eg;
+}
+
 // the context proper, from a block table whose ghost map is resolved; shard: the
 // exchange plan of a case split over ranks (nullptr otherwise)
 static int create_impl(const std::vector<mbm_block_desc>& glob, const std::vector<int>& blk_case,
@@ -1061,6 +1099,9 @@ static int create_impl(const std::vector<mbm_block_desc>& glob, const std::vecto
     // the grid barrier, so that the others' bounded waits (20 ms then) run out
     const char* drop = getenv("MBM_TILE_TEST_DROP");
     c->tile_drop = drop && atoi(drop) == 1;
+    // test hook: a grid for more CTAs per SM than are resident, which the launch refuses
+    const char* over = getenv("MBM_TILE_TEST_CTAS");
+    if (over && atoi(over) > 0) c->tile_grid = (int)std::min<long long>(tiles, (long long)c->nsm * atoi(over));
   }
   c->max_items = std::max<long long>(1, max_items);
   CKC(cudaMalloc(&c->dwork, sizeof(Work) * 2 * c->max_items));
@@ -1107,43 +1148,7 @@ static int create_impl(const std::vector<mbm_block_desc>& glob, const std::vecto
     const char* pe = getenv("MBM_PDL");
     c->pdl = !(pe && atoi(pe) == 0);
   }
-  // the step loop: while (any case live) { stage 1; fill TMP; stage 2; fill NEW; control }
-  // (in tiles without checkpoints: tile_steps)
-  if (!c->tile_loop) {
-    auto build_graph = [&]() -> cudaError_t {
-      cudaError_t e;
-      cudaGraphConditionalHandle h;
-      if ((e = cudaGraphCreate(&c->graph, 0))) return e;
-      if ((e = cudaGraphConditionalHandleCreate(&h, c->graph, 1, cudaGraphCondAssignDefault))) return e;
-      cudaGraphNodeParams np = {};
-      np.type = cudaGraphNodeTypeConditional;
-      np.conditional.handle = h;
-      np.conditional.type = cudaGraphCondTypeWhile;
-      np.conditional.size = 1;
-      cudaGraphNode_t node;
-      if ((e = cudaGraphAddNode(&node, c->graph, nullptr, 0, &np))) return e;
-      cudaGraph_t body = np.conditional.phGraph_out[0];
-      if ((e = cudaStreamBeginCaptureToGraph(c->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)))
-        return e;
-      const cudaError_t e1 = launch_attempt(c, h, 1);
-      cudaGraph_t captured = nullptr;
-      const cudaError_t e2 = cudaStreamEndCapture(c->stream, &captured);
-      if (e1) return e1;
-      if (e2) return e2;
-      return cudaGraphInstantiate(&c->gexec, c->graph, 0);
-    };
-    cudaError_t eg = build_graph();
-    if (eg != cudaSuccess && c->pdl) {   // without programmatic launches, once more
-      if (c->gexec) cudaGraphExecDestroy(c->gexec);
-      if (c->graph) cudaGraphDestroy(c->graph);
-      c->gexec = nullptr;
-      c->graph = nullptr;
-      cudaGetLastError();
-      c->pdl = false;
-      eg = build_graph();
-    }
-    CKC(eg);
-  }
+  if (!c->tile_loop) CKC(step_graph(c));
   int st = wait_stream(c);
   if (st != MBM_OK) return bail(st);
   *out = c;
@@ -1453,10 +1458,21 @@ extern "C" int mbm_steps_batch_async(mbm_ctx* c, const double* t, const double* 
     L.wait_ns = c->tile_drop ? 20000000ull : TILE_WAIT_NS;
     c->tile_drop = 0;
     CK(cudaMemsetAsync(c->dsync, 0, tile_scratch(c), c->stream));
-    CK(c->fast ? fastmath::launch_tile_steps(L, c->tile_grid, c->stream)
-               : bitwise::launch_tile_steps(L, c->tile_grid, c->stream));
-    CK(cudaMemcpyAsync(c->hsync, c->dsync + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
-  } else if (any && !c->host_loop) {
+    const cudaError_t e = c->fast ? fastmath::launch_tile_steps(L, c->tile_grid, c->stream)
+                                  : bitwise::launch_tile_steps(L, c->tile_grid, c->stream);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+      // this process may use fewer SMs than the device reports (a shared device): the graph's
+      // kernels need no residency
+      cudaGetLastError();
+      CK(step_graph(c));
+      c->tile_loop = false;
+    } else {
+      CK(e);
+      CK(cudaMemcpyAsync(c->hsync, c->dsync + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+      return MBM_OK;
+    }
+  }
+  if (any && !c->host_loop) {
     CK(cudaMemsetAsync(c->dqueue, 0, sizeof(int) * 10, c->stream));
     CK(cudaGraphLaunch(c->gexec, c->stream));
   } else if (any) {
