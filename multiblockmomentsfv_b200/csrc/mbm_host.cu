@@ -1954,8 +1954,13 @@ extern "C" int mbm_replay(mbm_ctx* c, const double* dts, int n, double* J) {
     CK(cudaMalloc(&c->adj_dtrep, sizeof(double) * n));
     c->adj_nrep = n;
   }
-  if (n > 0) CK(cudaMemcpyAsync(c->adj_dtrep, dts, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
-  if ((st = frozen_begin(c))) return st;     // also orders the dt copy before the host returns
+  if (n > 0) {      // the caller's array is done with here, whatever it is and however the call ends
+    void* r;
+    if ((st = ring_put(c, dts, sizeof(double) * n, &r))) return st;
+    CK(cudaMemcpyAsync(c->adj_dtrep, r ? r : dts, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
+    if (!r && (st = wait_stream(c))) return st;
+  }
+  if ((st = frozen_begin(c))) return st;
   for (int k = 0; k < n; k++) {
     if ((st = frozen_step(c, c->buf[cur], c->buf[1 - cur], c->adj_dtrep + k, c->buf[2]))) return st;
     cur = 1 - cur;

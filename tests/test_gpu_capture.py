@@ -29,6 +29,7 @@ CALLS = {
     "set_physics": lambda s, U, p: s._check(s.L.mbm_set_physics(s.ctx, C.c_double(0.1), C.c_double(0.0))),
     "steps_async": lambda s, U, p: s._check(s.L.mbm_steps_batch_async(
         s.ctx, (C.c_double * 1)(0.0), (C.c_double * 1)(1.0), C.c_double(1.0), C.c_double(0.9), 3)),
+    "replay": lambda s, U, p: s._check(s.L.mbm_replay(s.ctx, (C.c_double * 1)(1e-4), 1, None)),
 }
 
 

@@ -71,3 +71,30 @@ def test_a_wait_for_room_that_runs_out_is_reported(monkeypatch, ncase):
         _abi.check(s.L.mbm_set_physics(s.ctx, 0.02, 0.0), s.ctx)
         t, n, _ = s.steps(0.0, 1.0, max_steps=2)
         assert np.all(n == 2)
+
+
+@pytest.mark.parametrize("mode", ["exact", "fast"])
+def test_replayed_steps_on_both_sides_of_the_ring(mode):
+    """mbm_replay with more time steps than go through the ring, from page-locked memory, against the
+    same steps a part at a time: the same layers, and the same dt however they reach the device."""
+    import ctypes as C
+
+    import torch
+    from multiblockmomentsfv_b200 import scenario as sc
+    d = bf.Deck(Kn=0.05, limiter=4)
+    d.blocks = [bf.Block(1, -1.0, 1.0, -1.0, 1.0, 9, 8, (0, 0, 0, 0))]
+    n = 14500                                     # 116,000 bytes; the ring takes 114,688
+    dts = torch.from_numpy(np.random.default_rng(4).uniform(1e-6, 4e-6, n)).pin_memory()
+    out = []
+    for parts in ([n], [5000, 1, 9499]):
+        with sv.Solver(d, sc.Scenario.seeded_quadrant(6), mode=mode) as s:
+            s.initialise()
+            at = 0
+            for k in parts:
+                p = C.cast(dts.data_ptr() + 8 * at, C.POINTER(C.c_double))
+                s._check(s.L.mbm_replay(s.ctx, p, k, None))
+                at += k
+            assert at == n
+            out.append(s.download(0, 0))
+    H.assert_bitwise(out[0], out[1], "layer")
+    assert np.isfinite(out[0]).all()
