@@ -33,10 +33,11 @@ __global__ void ghost_kernel(const BlockDev* __restrict__ blk, const CaseDev* __
 // one Steps iteration's bookkeeping (control_cases, mbm_step.cuh)
 __global__ void control_kernel(CaseDev* cases, int ncases, const BlockDev* __restrict__ blk,
                                unsigned long long* lam, double* trace, int* queues,
-                               cudaGraphConditionalHandle h, int use_handle, const double* cfl_ext, int width) {
+                               cudaGraphConditionalHandle h, int use_handle, const double* cfl_ext,
+                               int lanes_log2) {
   pdl_enter();
   if (threadIdx.x < 10) queues[threadIdx.x] = 0;  // work counters [stage][limiter]
-  const int live = control_cases(cases, ncases, blk, lam, trace, cfl_ext, width);
+  const int live = control_cases(cases, ncases, blk, lam, trace, cfl_ext, lanes_log2);
   if (use_handle && threadIdx.x == 0) cudaGraphSetConditional(h, live ? 1u : 0u);
 }
 
@@ -286,7 +287,8 @@ cudaError_t launch_shard_cfl(const CaseDev* cases, const BlockDev* blk, int nblk
 
 cudaError_t launch_control_ext(CaseDev* cases, const BlockDev* blk, unsigned long long* lam, double* trace,
                                int* queues, const double* cfl_ext, cudaStream_t s) {
-  control_kernel<<<1, 256, 0, s>>>(cases, 1, blk, lam, trace, queues, cudaGraphConditionalHandle{}, 0, cfl_ext, 32);
+  control_kernel<<<1, CONTROL_THREADS, 0, s>>>(cases, 1, blk, lam, trace, queues, cudaGraphConditionalHandle{}, 0,
+                                               cfl_ext, 5);
   return cudaGetLastError();
 }
 
@@ -302,8 +304,8 @@ cudaError_t launch_ghost(const BlockDev* blk, const CaseDev* cases, const GhostE
 cudaError_t launch_control(CaseDev* cases, int ncases, const BlockDev* blk, int nblk, unsigned long long* lam,
                            double* trace, int* queues, cudaGraphConditionalHandle h, int use_handle,
                            cudaStream_t s) {
-  return launch_k(control_kernel, dim3(1), dim3(256), 0, s, cases, ncases, blk, lam, trace, queues, h, use_handle,
-                  (const double*)nullptr, control_width(ncases, nblk));
+  return launch_k(control_kernel, dim3(1), dim3(CONTROL_THREADS), 0, s, cases, ncases, blk, lam, trace, queues, h,
+                  use_handle, (const double*)nullptr, control_lanes_log2(ncases, nblk));
 }
 
 cudaError_t launch_stage_cfl(const BlockDev* blk, int nblk, const CaseDev* cases,

@@ -115,25 +115,28 @@ __device__ __forceinline__ void control_case(CaseDev& cs, double cfl, double* tr
   }
 }
 
-// the lanes of a case's controller: the cases' mean number of blocks, up to a power of two, at most 32
-inline int control_width(int ncases, int nblk) {
-  int w = 1;
-  while (w < 32 && (long long)w * ncases < nblk) w *= 2;
-  return w;
+// The controllers' one CTA, and the lanes of each case's, as a power of two: up to a warp while
+// they fit the CTA side by side, and no fewer than the cases have blocks on average.
+constexpr int CONTROL_THREADS = 256;
+
+inline int control_lanes_log2(int ncases, int nblk) {
+  int k = 5;
+  while (k > 0 && (long long)ncases << k > CONTROL_THREADS && (long long)ncases << (k - 1) >= nblk) k--;
+  return k;
 }
 
 // The controllers of every case, called by all threads of one CTA; clears the maxima.  Returns,
-// in every thread, whether a case is still live.  A case gets `width` lanes (control_width): one
-// case of 28 blocks a warp, a batch of one-block cases a thread each.  A chain of dependent loads and divisions per case, 2.4 us, is
-// what bounds it, so many cases must run side by side: a step attempt of 512 one-block cases of
-// 24^2 cells, fast, 279 us with a warp per case, 124 like this.
+// in every thread, whether a case is still live.  A case gets 1 << lanes_log2 lanes: one case a
+// warp, a batch of 512 one-block cases a thread each.  A chain of dependent loads and divisions,
+// 2.4 us a case, is what bounds it, so many cases must run side by side: a step attempt of 512
+// one-block cases of 24^2 cells, fast, 279 us with a warp per case, 124 like this.
 __device__ __forceinline__ int control_cases(CaseDev* cases, int ncases, const BlockDev* __restrict__ blk,
                                              unsigned long long* lam, double* trace, const double* cfl_ext,
-                                             int width) {
+                                             int lanes_log2) {
   int live = 0;
-  const int lane = threadIdx.x & (width - 1);
+  const int width = 1 << lanes_log2, lane = threadIdx.x & (width - 1);
   const unsigned mask = (width == 32 ? 0xffffffffu : (1u << width) - 1u) << (threadIdx.x & 31 & ~(width - 1));
-  for (int c = threadIdx.x / width; c < ncases; c += blockDim.x / width) {
+  for (int c = threadIdx.x >> lanes_log2; c < ncases; c += blockDim.x >> lanes_log2) {
     CaseDev& cs = cases[c];
     if (cs.done) continue;
     bool flagged;      // (never here: the stages' kernels flag cs.nonfinite)

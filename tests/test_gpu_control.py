@@ -22,9 +22,9 @@ def _case(k, nblocks, n):
     return d, sc.Scenario.seeded_quadrant(k)
 
 
-# mean blocks a case 1; 1.2, 2.5, 5, 11, 20, 40 with the cases' own counts far on either side
-@pytest.mark.parametrize("counts", [[1] * 300, [1] * 38 + [9], [1, 4] * 9, [1, 9, 2, 8] * 2, [33, 1, 7, 3],
-                                    [33, 7], [40]])
+# 1, 2, 4, 8, 16 and 32 lanes a case, with the cases' numbers of blocks on either side of that
+@pytest.mark.parametrize("counts", [[1] * 300, [1] * 99 + [7], [1] * 38 + [9], [1, 4] * 9, [1, 9, 2, 8, 1, 33] * 2,
+                                    [1, 9, 2, 8] * 2, [33, 1, 7, 3], [33, 7], [40]])
 def test_widths(counts, monkeypatch):
     cases = [_case(k, nb, 6) for k, nb in enumerate(counts)]
     tend = np.array([0.002 * (1 + k % 3) for k in range(len(counts))])
