@@ -311,7 +311,7 @@ __device__ __forceinline__ bool stage_item(const StageArgs& a, const Work w, con
     }
     cp_async_commit();
   };
-  u_fetch(rs);
+  if constexpr (TMA) u_fetch(rs);
   d0_fetch(rs - 2);
   double Un[NV];
   const int Cin = min(max(C, 0), nxp - 1);   // lanes and rows outside the grid: the nearest cell's values, unused
