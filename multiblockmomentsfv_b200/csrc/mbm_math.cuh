@@ -37,11 +37,11 @@ __device__ __forceinline__ double rsgn(double a) { return a == 0 ? 0.0 : (a < 0 
 // Reciprocal, square root and lone quotients.  Bitwise: the exact division of mbm_div.cuh,
 // IEEE division and sqrt.
 //
-// Fast arithmetic (MBM_FAST_ARITH, MBM_MODE_FAST): the quotient is RN(x*r) without
-// the correction, within one unit in the last place of x/y, and nothing is checked.  Its
-// multiply-adds are written out, not left to the compiler's contraction, so that every
-// kernel that evaluates these functions (row march, tiles) gets the same bits.
-// Fast arithmetic: the refined hardware approximations of mbm_newton.cuh.
+// Fast arithmetic (MBM_FAST_ARITH, MBM_MODE_FAST): the refined hardware approximations of
+// mbm_newton.cuh; the quotient is RN(x*r) without the correction, within one unit in the last
+// place of x/y, and nothing is checked.  Its multiply-adds are written out, not left to the
+// compiler's contraction, so that every kernel that evaluates these functions (row march, tiles)
+// gets the same bits.
 #if MBM_FAST_ARITH
 using mbm_newton::frcp;
 using mbm_newton::fsqrt;
@@ -181,50 +181,6 @@ __device__ __forceinline__ void grad13_flux_x(const double (&U)[NV], double (&F)
          rho * (M111 * v1 + M112 * v2) + 0.5 * rho * (T11 * vs + R11);
   F[8] = q2 * v1 + q1 * v2 + rho * (v1 * v2 * (T11 + T22) + 1.5 * T12 * vs) + E * v1 * v2 +
          rho * (M121 * v1 + M122 * v2) + 0.5 * rho * R12;
-}
-
-// a*c + b*d with one of c, d +-1 and the other +-0, as the rotations of the flux need it:
-// the product with +-1 is exact, so one FMA rounds like the two products and the sum
-// (signs of zeros included) at a third of the operations
-__device__ __forceinline__ double rot(double a, double c, double b, double d) {
-  return (c == 1.0 || c == -1.0) ? fma(b, d, c == 1.0 ? a : -a) : fma(a, c, d == 1.0 ? b : -b);
-}
-
-// flux through a face of unit normal (nx, ny): rotate, x-flux, rotate back
-// (src/Flux.c:126-172).  The products with 0 are kept (in FMAs): they fix the
-// signs of zeros exactly as the reference computes them.
-template <int DIR>
-__device__ __forceinline__ void flux_normal(const double (&U)[NV], double (&F)[NV]) {
-  constexpr double nx = DIR == 1 ? 1.0 : 0.0, ny = DIR == 1 ? 0.0 : 1.0;
-  constexpr double tx = ny, ty = -nx;
-  double W[NV], G[NV], a, b;
-  W[0] = U[0];
-  W[1] = rot(U[1], nx, U[2], ny);
-  W[2] = rot(U[1], tx, U[2], ty);
-  W[3] = U[3];
-  a = rot(U[4], nx, U[5], ny);
-  b = rot(U[5], nx, U[6], ny);
-  W[4] = rot(a, nx, b, ny);
-  W[5] = rot(a, tx, b, ty);
-  a = rot(U[4], tx, U[5], ty);
-  b = rot(U[5], tx, U[6], ty);
-  W[6] = rot(a, tx, b, ty);
-  W[7] = rot(U[7], nx, U[8], ny);
-  W[8] = rot(U[7], tx, U[8], ty);
-  grad13_flux_x(W, G);
-  F[0] = G[0];
-  F[1] = rot(G[1], nx, G[2], tx);
-  F[2] = rot(G[1], ny, G[2], ty);
-  F[3] = G[3];
-  a = rot(G[4], nx, G[5], tx);
-  b = rot(G[5], nx, G[6], tx);
-  F[4] = rot(a, nx, b, tx);
-  F[5] = rot(a, ny, b, ty);
-  a = rot(G[4], ny, G[5], ty);
-  b = rot(G[5], ny, G[6], ty);
-  F[6] = rot(a, ny, b, ty);
-  F[7] = rot(G[7], nx, G[8], tx);
-  F[8] = rot(G[7], ny, G[8], ty);
 }
 #endif
 
@@ -539,7 +495,7 @@ __device__ __forceinline__ void cons_flux_x(const double (&P)[NV], double (&U)[N
 //   (lamR fL - lamL fR + lamL lamR (UR - UL)) / alpha
 // come first, then each side's moments and flux are formed and added in turn, so one
 // side's vectors are live at a time (alpha = 0, both speeds 0: the mean of the two
-// fluxes, coefficients 1/2, -1/2, 0).  Mathematically the bitwise version below; the
+// fluxes, coefficients 1/2, -1/2, 0).  Mathematically hll_swapped below; the
 // rounding differs.
 template <int DIR>
 __device__ __forceinline__ double hll(const double (&PL_)[NV], const double (&PR_)[NV],
@@ -579,55 +535,19 @@ __device__ __forceinline__ double hll(const double (&PL_)[NV], const double (&PR
   return cMax;
 }
 #else
-// FnumHLLE (src/Flux.c:308-379) for a face with left/right primitives.
-// DIR = 1: x face (normal (1,0)), DIR = 2: y face (normal (0,1)).  The
-// diffusive scale FFlux/GFlux return is 0, so lamDiff(0/(cMax*dx)) is 1 for
-// every cMax and cMax/1.0 == cMax: the division is omitted without changing a bit.
-// The left side is reduced to lamR fL and UL before the right side is formed, so that one
-// side's vectors are live at a time (alpha <= 0: the mean of the fluxes, with factor 1 in
-// place of lamR).
-template <int DIR>
-__device__ __forceinline__ double hll(const double (&PL)[NV], const double (&PR)[NV],
-                                      double (&flx)[NV]) {
-  const double cR = 2.0 * sqrt(5.0 / 3 * PR[3]);
-  const double cL = 2.0 * sqrt(5.0 / 3 * PL[3]);
-  const double vR = PR[DIR], vL = PL[DIR];
-  const double cMax = fabs(0.5 * (vL + vR)) + rmax(cR, cL);
-  const double lamL = rmin(vL - cL, 0.0);
-  const double lamR = rmax(vR + cR, 0.0);
-  const double alph = lamR - lamL;
-  const bool pos = alph > 0.0;
-  double UL[NV], UR[NV], f[NV], A[NV];
-  conservative(PL, UL);
-  flux_normal<DIR>(UL, f);
-  const double kL = pos ? lamR : 1.0;
-#pragma unroll
-  for (int n = 0; n < NV; n++) A[n] = kL * f[n];
-  conservative(PR, UR);
-  flux_normal<DIR>(UR, f);
-  if (pos) {
-    const Recip D(alph);
-    double num[NV];
-#pragma unroll
-    for (int n = 0; n < NV; n++) num[n] = A[n] - lamL * f[n] + lamL * lamR * (UR[n] - UL[n]);
-    quotients(num, D, flx);
-  } else {
-#pragma unroll
-    for (int n = 0; n < NV; n++) flx[n] = 0.5 * (A[n] + f[n]);
-  }
-  return cMax;
-}
 // v, or -v where sg is the sign bit
 __device__ __forceinline__ double signed_by(double v, unsigned sg) {
   return __hiloint2double(__double2hiint(v) ^ (int)sg, __double2loint(v));
 }
 
-// flux_normal with the direction a run-time value: U and F of a y face come with x and y
-// swapped, so that both directions run the same operations.  An x face rotates by normal
-// (1, 0), tangent (0, -1), a y face by (0, 1), (1, -0): in the swapped order the two differ by
-// the sign of the second component (sg: the sign bit for x faces) and by the sign of the zero
-// products (z: +0 for x, -0 for y faces), each FMA below being the one that flux_normal
-// forms in its direction.
+// Flux through a face: rotate to the normal, x-flux, rotate back (src/Flux.c:126-172), with the
+// direction a run-time value: U and F of a y face come with x and y swapped, so that both
+// directions run the same operations.  The reference forms each rotated component as a*c + b*d
+// with one of c, d +-1 and the other +-0; the product with +-1 is exact, so one FMA rounds like
+// the two products and the sum (signs of zeros included).  An x face has normal (1, 0) and
+// tangent (0, -1), a y face (0, 1) and (1, -0): in the swapped order the two differ by the sign of
+// the second component (sg: the sign bit for x faces) and by the sign of the zero products (z:
+// +0 for x, -0 for y faces), which fix the signs of zeros as the reference computes them.
 __device__ __forceinline__ void flux_swapped(const double (&U)[NV], bool y, unsigned sg, double z,
                                              double (&F)[NV]) {
   double W[NV], G[NV];
@@ -658,8 +578,12 @@ __device__ __forceinline__ void flux_swapped(const double (&U)[NV], bool y, unsi
   F[8] = fma(G[7], 0.0, signed_by(G[8], sg));
 }
 
-// hll with the direction a run-time value: states and flux of a y face with x and y swapped
-// (Conservative commutes with the swap bit for bit)
+// FnumHLLE (src/Flux.c:308-379) for a face with left/right primitives, the direction a run-time
+// value: states and flux of a y face with x and y swapped (Conservative commutes with the swap
+// bit for bit).  The diffusive scale FFlux/GFlux return is 0, so lamDiff(0/(cMax*dx)) is 1 for
+// every cMax and cMax/1.0 == cMax: the division is omitted without changing a bit.  The left
+// side is reduced to lamR fL and UL before the right side is formed, so that one side's vectors
+// are live at a time (alpha <= 0: the mean of the fluxes, with factor 1 in place of lamR).
 __device__ __forceinline__ double hll_swapped(const double (&PL)[NV], const double (&PR)[NV], bool y,
                                               double (&flx)[NV]) {
   const unsigned sg = y ? 0u : 0x80000000u;
