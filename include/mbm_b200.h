@@ -205,6 +205,11 @@ int mbm_case_status(mbm_ctx *ctx, int *status, int n);
  * rounded results.  Normal positive operands. */
 int mbm_fastmath_check(const double *x, int n, double *out);
 
+/* The same for the bitwise kernels' divisions of n pairs in device memory (no counterpart in
+ * the reference): out (device, 3n doubles) receives x/y by itself, x/y as one of a set that shares
+ * the reciprocal of y, and the harmonic limiter's slope of (x[i], x[i+1]) over y. */
+int mbm_division_check(const double *x, const double *y, int n, double *out);
+
 /* ---- One case split over ranks by block (one process per GPU) ----------------
  * No counterpart in the reference, which runs every block in one process.  Each
  * rank owns whole blocks (owner[b] = rank of block b, the same table on every

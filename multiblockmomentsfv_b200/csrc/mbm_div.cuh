@@ -24,8 +24,9 @@
 // limiter, 1.81 ms like this; 28 blocks of 30 x 10 in a stream, most sets holding a zero,
 // 143 against 129 us (checking exponents alone and sorting the zeros out in a second look:
 // 1.96 ms and 143 us).
-// Checked against x/y on the host for random and near-tie operands
-// (tests/test_division.py, tests/test_exact_division.py) and by every bitwise parity test.
+// Checked against x/y, restated on the host (tests/test_exact_division.py) and on the device
+// as it stands (tests/test_gpu_division.py: zeros of both signs, significands of all ones, near
+// ties, the edges of the admitted range and what is outside it), and by every bitwise parity test.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -328,4 +328,29 @@ cudaError_t launch_planes_to_aos(const double* src, double* aos, int nxp, int ny
   return cudaGetLastError();
 }
 
+// what the stages divide with, of n pairs: a quotient by itself, one of a set of three by a
+// shared reciprocal, and the harmonic limiter's slope
+__global__ void division_check_kernel(const double* __restrict__ x, const double* __restrict__ y, int n,
+                                      double* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double a = x[i], b = x[(i + 1) % n], c = x[(i + 2) % n], d = y[i];
+  const Recip D(d);
+  double q[3], S[1];
+  quotients({a, b, c}, D, q);
+  slopes<4>({a}, {b}, D, S);
+  out[3 * (size_t)i] = div_rn(a, d);
+  out[3 * (size_t)i + 1] = q[0];
+  out[3 * (size_t)i + 2] = S[0];
+}
+
 }  // namespace mbm
+
+// The bitwise kernels' divisions of n pairs (device values; out: 3n), for checking them
+// against IEEE division.
+extern "C" int mbm_division_check(const double* x, const double* y, int n, double* out) {
+  if (!x || !y || !out || n < 0) return 1;   // MBM_EINVAL
+  if (n == 0) return 0;
+  mbm::division_check_kernel<<<(n + 255) / 256, 256>>>(x, y, n, out);
+  return cudaDeviceSynchronize() == cudaSuccess ? 0 : 4;   // MBM_OK / MBM_ECUDA
+}
