@@ -93,7 +93,7 @@ int mbm_destroy(mbm_ctx *ctx);
 /* Many independent cases in one context (no counterpart in the reference, which
  * runs one case per process): every Heun stage of every case is one persistent
  * launch, and mbm_steps_batch advances all cases together in
- * one CUDA-graph loop, each with its own dt, t and step count.  Blocks are indexed
+ * one CUDA-graph loop (small grids: one kernel), each with its own dt, t and step count.  Blocks are indexed
  * globally in the transfer calls. */
 int mbm_create_batch(const mbm_block_desc *blocks, int nblocks, const mbm_case_desc *cases,
                      int ncases, const mbm_params *params, mbm_ctx **ctx);
@@ -194,7 +194,8 @@ int mbm_attempts(mbm_ctx *ctx, int *attempts);
 
 /* Status of each of the first n cases after the last step-loop call: MBM_OK, or
  * MBM_ENONFINITE (the case stopped at the attempt that produced a NaN or infinity;
- * its state is the last accepted one) or MBM_ESTEPLIMIT.  The call itself returned
+ * its state is the last accepted one), MBM_ESTEPLIMIT or MBM_ETIMEOUT (a bounded wait on
+ * the device ran out).  The call itself returned
  * the worst of them; the other cases ran to the end.  No counterpart in the
  * reference, whose loop runs on through non-finite values. */
 int mbm_case_status(mbm_ctx *ctx, int *status, int n);

@@ -443,8 +443,9 @@ __global__ void __launch_bounds__(32 * GWARPS) adj_gather(AdjArgs a, const doubl
 // update's relaxation term (the Data0 term is in pass A)
 #ifndef ADJ_POINT_CTAS
 // resident 128-thread CTAs per SM the pointwise pass is compiled for: a cell's loads are all
-// asked for at the start, so four without spills keep enough of them in flight and ran the
-// reverse sweep of 60 steps at 4 x 256^2 in 18.0 ms, six (64 bytes of spills) in 18.3.  The
+// asked for at the start, so four (117 registers in stage 2, no spills; 128 and 48 bytes of
+// spills in stage 1) keep enough of them in flight and ran the reverse sweep of 60 steps at 4 x
+// 256^2 in 18.0 ms, six (64 bytes of spills) in 18.3.  The
 // pass takes 26 us; with the loads of a layer asked for where it is used it took 36.
 #define ADJ_POINT_CTAS 4
 #endif

@@ -136,7 +136,7 @@ struct mbm_ctx {
   CaseDev* dcase = nullptr;
   CaseDev* hcase = nullptr;         // pinned mirror, ncase entries
   unsigned long long* dlam = nullptr;
-  int* dqueue = nullptr;            // work counters [stage][limiter]
+  int* dqueue = nullptr;            // the work counters of the two stages' launches
   double* dtrace = nullptr;
   double* dcfl = nullptr;           // per-block stage CFL for mbm_update
   double* hcfl = nullptr;           // pinned
@@ -535,7 +535,7 @@ static cudaError_t launch_stages(mbm_ctx* c, int heun, int sel_in, int sel_d0, i
   StageArgs a = stage_args(c, heun, bufs);
   a.work = c->dwork + heun * c->max_items;
   a.nwork = c->nwork[heun];
-  a.queue = c->dqueue + heun * 5;
+  a.queue = c->dqueue + heun;
   a.sel_in = sel_in; a.sel_d0 = sel_d0; a.sel_out = sel_out;
   a.rlx_read = heun == 1 && rlx_read;
   // bulk tensor copies: fast stage 2 on the context's own layers (the maps cover TMP
@@ -605,13 +605,13 @@ static std::map<std::tuple<long long, int, int, int>, std::array<double, 2>> g_t
 // then two timed launches of each stage
 static int time_each_stage(mbm_ctx* c, cudaEvent_t e0, cudaEvent_t e1, float* ms) {
   for (int heun = 0; heun < 2; heun++) {
-    CK(cudaMemsetAsync(c->dqueue, 0, sizeof(int) * 10, c->stream));
+    CK(cudaMemsetAsync(c->dqueue, 0, sizeof(int) * 2, c->stream));
     CK(launch_stages(c, heun, heun ? SEL_TMP : SEL_CUR, SEL_CUR, heun ? SEL_OTHER : SEL_TMP, 1));
   }
   for (int heun = 0; heun < 2; heun++) {
     CK(cudaEventRecord(e0, c->stream));
     for (int rep = 0; rep < 2; rep++) {
-      CK(cudaMemsetAsync(c->dqueue, 0, sizeof(int) * 10, c->stream));
+      CK(cudaMemsetAsync(c->dqueue, 0, sizeof(int) * 2, c->stream));
       CK(launch_stages(c, heun, heun ? SEL_TMP : SEL_CUR, SEL_CUR, heun ? SEL_OTHER : SEL_TMP, 1));
     }
     CK(cudaEventRecord(e1, c->stream));
@@ -1071,8 +1071,8 @@ static int create_impl(const std::vector<mbm_block_desc>& glob, const std::vecto
     c->lim = k == 0 || h.limiter == c->lim ? h.limiter : LIM_ANY;
   }
   CKC(cudaMemcpyAsync(c->dcase, c->hcase, sizeof(CaseDev) * ncases, cudaMemcpyHostToDevice, c->stream));
-  CKC(cudaMalloc(&c->dqueue, sizeof(int) * 10));
-  CKC(cudaMemsetAsync(c->dqueue, 0, sizeof(int) * 10, c->stream));
+  CKC(cudaMalloc(&c->dqueue, sizeof(int) * 2));
+  CKC(cudaMemsetAsync(c->dqueue, 0, sizeof(int) * 2, c->stream));
   CKC(cudaMalloc(&c->dlam, sizeof(unsigned long long) * 6 * nblocks));
   CKC(cudaMemsetAsync(c->dlam, 0, sizeof(unsigned long long) * 6 * nblocks, c->stream));
   CKC(cudaMalloc(&c->dtrace, sizeof(double) * 4 * MAX_TRACE * ncases));
@@ -1370,7 +1370,7 @@ extern "C" int mbm_set_boundary(mbm_ctx* c, int layer, double t) {
 
 static int run_stage(mbm_ctx* c, int out_layer, int in_layer, int d0_layer, int heun, double* cfl,
                      int rlx_read = 0) {
-  CK(cudaMemsetAsync(c->dqueue, 0, sizeof(int) * 10, c->stream));
+  CK(cudaMemsetAsync(c->dqueue, 0, sizeof(int) * 2, c->stream));
   CK(launch_stages(c, heun, layer_sel(in_layer), layer_sel(d0_layer), layer_sel(out_layer), rlx_read));
   CK(launch_stage_cfl(c->dblk, c->nblk, c->dcase, c->dlam, heun, c->dcfl, c->stream));
   CK(cudaMemcpyAsync(c->hcfl, c->dcfl, sizeof(double) * c->nblk, cudaMemcpyDeviceToHost, c->stream));
@@ -1473,13 +1473,13 @@ extern "C" int mbm_steps_batch_async(mbm_ctx* c, const double* t, const double* 
     }
   }
   if (any && !c->host_loop) {
-    CK(cudaMemsetAsync(c->dqueue, 0, sizeof(int) * 10, c->stream));
+    CK(cudaMemsetAsync(c->dqueue, 0, sizeof(int) * 2, c->stream));
     CK(cudaGraphLaunch(c->gexec, c->stream));
   } else if (any) {
     // the graph body launched from the host, 16 attempts between checks of the
     // controller state (kernels of finished cases return at once); for tools that
     // cannot look inside conditional graph nodes
-    CK(cudaMemsetAsync(c->dqueue, 0, sizeof(int) * 10, c->stream));
+    CK(cudaMemsetAsync(c->dqueue, 0, sizeof(int) * 2, c->stream));
     for (;;) {
       for (int k = 0; k < 16; k++) CK(launch_attempt(c, 0, 0));
       CK(cudaMemcpyAsync(c->hcase, c->dcase, sizeof(CaseDev) * c->ncase, cudaMemcpyDeviceToHost, c->stream));
@@ -1610,12 +1610,12 @@ extern "C" int mbm_time_stage(mbm_ctx* c, int heun, double dt, int reps, double*
   cudaEvent_t& e1 = ev.e[1];
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
-  CK(cudaMemsetAsync(c->dqueue, 0, sizeof(int) * 10, c->stream));
+  CK(cudaMemsetAsync(c->dqueue, 0, sizeof(int) * 2, c->stream));
   CK(launch_stages(c, heun, si, SEL_CUR, so, 1));      // warm-up launch
-  // the per-launch queue reset is a 40-byte memset, inside the timed region
+  // the per-launch queue reset is an 8-byte memset, inside the timed region
   CK(cudaEventRecord(e0, c->stream));
   for (int r = 0; r < reps; r++) {
-    CK(cudaMemsetAsync(c->dqueue, 0, sizeof(int) * 10, c->stream));
+    CK(cudaMemsetAsync(c->dqueue, 0, sizeof(int) * 2, c->stream));
     CK(launch_stages(c, heun, si, SEL_CUR, so, 1));
   }
   CK(cudaEventRecord(e1, c->stream));
@@ -2188,7 +2188,7 @@ extern "C" int mbm_shard_stage(mbm_ctx* c, int heun) {
   if (st) return st;
   if (heun != 0 && heun != 1) return fail(c, MBM_EINVAL, "mbm_shard_stage: bad argument");
   CK(cudaSetDevice(c->device));
-  CK(cudaMemsetAsync(c->dqueue + heun * 5, 0, sizeof(int) * 5, c->stream));
+  CK(cudaMemsetAsync(c->dqueue + heun, 0, sizeof(int), c->stream));
   CK(launch_stages(c, heun, heun ? SEL_TMP : SEL_CUR, SEL_CUR, heun ? SEL_OTHER : SEL_TMP, 1));
   return MBM_OK;
 }

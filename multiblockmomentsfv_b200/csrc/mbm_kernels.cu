@@ -36,7 +36,7 @@ __global__ void control_kernel(CaseDev* cases, int ncases, const BlockDev* __res
                                cudaGraphConditionalHandle h, int use_handle, const double* cfl_ext,
                                int lanes_log2) {
   pdl_enter();
-  if (threadIdx.x < 10) queues[threadIdx.x] = 0;  // work counters [stage][limiter]
+  if (threadIdx.x < 2) queues[threadIdx.x] = 0;  // the work counters of the two stages
   const int live = control_cases(cases, ncases, blk, lam, trace, cfl_ext, lanes_log2);
   if (use_handle && threadIdx.x == 0) cudaGraphSetConditional(h, live ? 1u : 0u);
 }
@@ -47,7 +47,7 @@ __global__ void control_kernel(CaseDev* cases, int ncases, const BlockDev* __res
 __global__ void frozen_prep_kernel(CaseDev* cases, const double* __restrict__ ddt, int* queues) {
   pdl_enter();
   if (threadIdx.x == 0) cases[0].dt = *ddt;
-  if (threadIdx.x < 10) queues[threadIdx.x] = 0;
+  if (threadIdx.x < 2) queues[threadIdx.x] = 0;
 }
 
 cudaError_t launch_frozen_prep(CaseDev* cases, const double* ddt, int* queues, cudaStream_t s) {

@@ -39,7 +39,7 @@ struct ExactWindow {
   double D0a[NV][32];       // stage 2: Data0 (or its stored relaxation term) of the row to be updated
 };
 
-// two CTAs of four warps per SM: 232 registers, no spills
+// two CTAs of four warps per SM: 240 to 254 registers, no spills
 constexpr int EXACT_WARPS = 4, EXACT_CTAS = 2;
 constexpr int EXACT_SMEM = (int)sizeof(ExactWindow) * EXACT_WARPS;
 

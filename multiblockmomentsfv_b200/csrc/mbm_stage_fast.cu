@@ -1,7 +1,8 @@
 // mbm_stage_fast.cu -- the Heun stage kernels in fast arithmetic (MBM_MODE_FAST):
-// the same kernel sources as the bitwise instantiation, with quotients from a shared
-// reciprocal without Markstein's correction and multiply-adds written out.  Results differ from the reference in the last
-// bits of single operations; the mode is held to the reference within 1e-10
+// the row march of mbm_stage.cuh (the bitwise one is mbm_stage_exact.cuh) and the tiles of
+// mbm_tile.cuh, with quotients from a shared reciprocal without Markstein's correction and
+// multiply-adds written out.  Results differ from the reference in the last bits of single
+// operations; the mode is held to the reference within 1e-10
 // relative per field after one step and 1e-8 at the end time.
 #define MBM_ARITH fastmath
 #define MBM_FAST_ARITH 1

@@ -21,6 +21,9 @@
 // TILE_MOST_* (mbm_internal.h), where both are measured.  What bounds it: with one tile per CTA
 // the chain through the four phases, 6,000 cycles fast and 14,000 bitwise per stage, and the
 // barrier over the grid, 2,500; with more, two CTAs per SM share the FP64 and issue slots.
+// Two CTAs per SM leave a thread 128 registers: 122 to 126 fast, no spills; bitwise 128 with 344
+// bytes of spill stores and 308 of loads in the step loop (one CTA per SM, without them, ran as
+// fast with one tile a CTA and slower with more).
 //
 // tile_steps runs whole Steps calls of such grids (src/Main.c:189-244): a cooperative grid
 // whose CTAs keep a few tiles each, with a barrier over the grid after each Heun stage.  The
