@@ -6,16 +6,16 @@
 // projected primitives of row r, the y slopes of row r-1 and the y-face flux between rows r-2
 // and r-1, then the x slopes and x-face fluxes of row r-2 and its update.
 //
-// The unfused, exactly rounded arithmetic takes 2,700 instructions a row where the fast mode
-// takes 1,450.  Written out straight, each direction with code of its own, a row is 44 KB of
-// instructions, more than an SM keeps close: its warps waited for instructions a fifth of the
-// time.  So the two directions are one loop, x and y swapped in the y pass (hll_swapped).  The
+// The unfused, exactly rounded arithmetic takes 126 M warp instructions a stage of 4 x 512^2 cells
+// where the fast mode takes 52 M.  Written out straight, each direction with code of its own, a
+// row is 44 KB of instructions, more than an SM keeps close: its warps waited for instructions a
+// fifth of the time.  So the two directions are one loop, x and y swapped in the y pass (hll_swapped).  The
 // moments of the next row and Data0 of the row to be updated are copied to shared memory
 // while a row is worked on (the next row's without a condition: lanes and rows outside the grid
 // copy the nearest cell), and the update's other term is loaded before the fluxes.
 //
-// What bounds it: fixed-latency dependencies and the FP64 pipe (40 % of its cycles) at two
-// warps per scheduler.  4 x 1024^2 cells, harmonic: 886 -> 815 us a stage (4 x 256^2: 78 ->
+// What bounds it: fixed-latency dependencies and the FP64 pipe (49 % of an SM's active cycles) at
+// two warps per scheduler.  4 x 1024^2 cells, harmonic: 886 -> 815 us a stage (4 x 256^2: 78 ->
 // 71); with copies under a condition and a state at rest in place of the missing cells 838,
 // without the copies 884; three warps per scheduler (168 registers; both sides of a face
 // one loop too, its states and partial sums in shared memory; no room for the copies, 20-100

@@ -20,7 +20,8 @@
 // and the fluxes 1.14 times (1.16), so large grids stay with the march; the line is drawn at
 // TILE_MOST_* (mbm_internal.h), where both are measured.  What bounds it: with one tile per CTA
 // the chain through the four phases, 6,000 cycles fast and 14,000 bitwise per stage, and the
-// barrier over the grid, 2,500; with more, two CTAs per SM share the FP64 and issue slots.
+// barrier over the grid, 2,500 (a step of 14 tiles: 21,200 and 34,000 cycles); with more, two
+// CTAs per SM share the FP64 and issue slots.
 // Two CTAs per SM leave a thread 128 registers: 122 to 126 fast, no spills; bitwise 128 with 344
 // bytes of spill stores and 308 of loads in the step loop (one CTA per SM, without them, ran as
 // fast with one tile a CTA and slower with more).
